@@ -10,42 +10,15 @@
 // Both are deterministic: every output's additions happen in an order that the inputs and the
 // launch shape fix.
 #include "deliver_pre.cuh"
+#include "fast_axis.cuh"
 
 #include <algorithm>
 
 namespace {
 
-using pvgpu::Axis;
+using pvgpu::fast_axis;
+using pvgpu::FastAxis;
 using pvgpu::PreGeom;
-
-// Axis::start as shifts: every legal ratio of layer sizes is a power of two (axis_legal), so
-// start(i) = (((i - c) << tl) >> sr) + o, the arithmetic shift being the floor of the many-to-one
-// case.  first_ge is its inverse in closed form (a binary search over start() cost each thread
-// about 2,000 cycles before the first entry was read).
-struct FastAxis {
-   int c, tl, sr, o, n;
-   __device__ __forceinline__ int start(int i) const { return (((i - c) << tl) >> sr) + o; }
-   // first i in [0, n] with start(i) >= v
-   __device__ __forceinline__ int first_ge(int v) const {
-      const int i = c + ((((v - o) << sr) + (1 << tl) - 1) >> tl);
-      return min(max(i, 0), n);
-   }
-};
-
-FastAxis fast_axis(const Axis &a, int nExt) {
-   auto log2i = [](int n) {
-      int s = 0;
-      while ((1 << s) < n) s++;
-      return s;
-   };
-   if (a.nPre == a.nPost) return FastAxis{a.preBorder + (a.patch - 1) / 2, 0, 0, 0, nExt};
-   if (a.nPre < a.nPost) {
-      const int t = a.nPost / a.nPre;
-      return FastAxis{a.preBorder, log2i(t), 0, -((a.patch - t) / 2), nExt};
-   }
-   const int s = a.nPre / a.nPost;
-   return FastAxis{a.preBorder + (s / 2) * (a.patch - 1), 0, log2i(s), 0, nExt};
-}
 
 struct FastGeom {
    FastAxis ax, ay;
