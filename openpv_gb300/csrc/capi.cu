@@ -19,6 +19,19 @@ pvgpu_status record_message(pvgpu_status status, const char *message) {
    return status;
 }
 
+int num_sms() {
+   static thread_local int device = -1, count = 0;
+   int dev = 0;
+   cudaGetDevice(&dev);
+   if (device != dev) {
+      int n = 0;
+      if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+      device = dev;
+      count = n;
+   }
+   return count;
+}
+
 }  // namespace pvgpu
 
 extern "C" const char *pvgpu_version(void) { return "pvgpu 0.1 (sm_103a)"; }

@@ -18,6 +18,7 @@ namespace {
 
 using pvgpu::fast_axis;
 using pvgpu::FastAxis;
+using pvgpu::num_sms;
 using pvgpu::PreGeom;
 
 struct FastGeom {
@@ -317,19 +318,6 @@ pvgpu_status launch_cols_nyp(const FastGeom &g, dim3 grid, int RS, cudaStream_t 
    }
 #undef PVGPU_NYP
    return PVGPU_ERR_UNSUPPORTED_SHAPE;
-}
-
-int num_sms() {
-   static thread_local int cached[2] = {-1, 0};
-   int dev = 0;
-   cudaGetDevice(&dev);
-   if (cached[0] != dev) {
-      int n = 0;
-      if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-      cached[0] = dev;
-      cached[1] = n;
-   }
-   return cached[1];
 }
 
 pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *entries, const int64_t *numActive,

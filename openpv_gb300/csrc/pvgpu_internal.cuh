@@ -25,6 +25,9 @@ pvgpu_status record_message(pvgpu_status status, const char *message);
       if (e_ != cudaSuccess) return ::pvgpu::record_cuda_error(e_, where);         \
    } while (0)
 
+// Streaming multiprocessors of the current device (148 where the query fails).
+int num_sms();
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Geometry of one layer, restated from include/PVLayerLoc.h and utils/conversions.hpp.
