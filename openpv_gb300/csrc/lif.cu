@@ -9,8 +9,11 @@
 // the per-launch decay factors exp(-dt/tau*) are computed on the host with the C library's expf
 // as the reference does; so 'b', whose per-neuron arithmetic has no transcendental, equals the
 // reference bit for bit, and 'a' / 'o' differ only by the device's expf / powf / logf (within a
-// few ulp) in their per-neuron filter coefficients.  Memory-bound: 88 bytes per neuron per step.
-#include "pvgpu_internal.cuh"
+// few ulp) in their per-neuron filter coefficients.  88 bytes per neuron per step: memory-bound, with
+// the arma coefficients (divisions and a powf per neuron) close behind.  A thread per neuron, blocks of
+// 256 in one grid: 255 us for 8 x 256x256x32, arma (5.8 TB/s, issue slots 78 % busy), against 310 us with 8 blocks an SM striding over the
+// layer (five fit, so the second round ran three fifths full) and four divisions to locate a neuron.
+#include "row_map.cuh"
 
 #include <cmath>
 
@@ -19,7 +22,8 @@ namespace {
 struct LifConst {
    pvgpu_lif_params p;
    float dt, dtSec, eE, eI, eIB, eVth;
-   int numNeurons, total, nx, ny, nf, lt, rt, dn, up, numExt;
+   int total;
+   pvgpu::RowMap map;
 };
 
 __device__ __forceinline__ uint32_t taus_component(uint32_t s, int a, int b, uint32_t mask, int d) {
@@ -72,10 +76,9 @@ __global__ void __launch_bounds__(256) lif_kernel(LifConst c, uint4 *__restrict_
                                                   const float *__restrict__ gsyn, float *__restrict__ aExt) {
    const float GMAX = 10.0f;
    const pvgpu_lif_params &p = c.p;
-   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < c.total; k += gridDim.x * blockDim.x) {
-      const int b = k / c.numNeurons, kr = k - b * c.numNeurons;
-      const int f = kr % c.nf, x = (kr / c.nf) % c.nx, y = kr / (c.nf * c.nx);
-      const int64_t kex = (int64_t)b * c.numExt + ((int64_t)(y + c.up) * (c.nx + c.lt + c.rt) + (x + c.lt)) * c.nf + f;
+   const int k = blockIdx.x * blockDim.x + threadIdx.x;
+   if (k < c.total) {
+      const int64_t kex = pvgpu::row_at<1, false>(c.map, k).ext;
       uint4 r = rnd[k];
       float v = V[k], vth = Vth[k], ge = GE[k], gi = GI[k], gib = GIB[k];
       const float inE = noise(r, gsyn[k], c.dtSec, p.noiseFreqE, p.noiseAmpE);
@@ -179,23 +182,15 @@ extern "C" pvgpu_status pvgpu_lif_update(const pvgpu_loc *loc, char method, cons
    c.eI = std::exp(-dt / params->tauI);
    c.eIB = std::exp(-dt / params->tauIB);
    c.eVth = std::exp(-dt / params->tauVth);
-   c.nx = loc->nx;
-   c.ny = loc->ny;
-   c.nf = loc->nf;
-   c.lt = loc->halo.lt;
-   c.rt = loc->halo.rt;
-   c.dn = loc->halo.dn;
-   c.up = loc->halo.up;
    const int64_t numNeurons = (int64_t)loc->nx * loc->ny * loc->nf;
    const int64_t total = numNeurons * loc->nbatch;
-   const int64_t numExt = (int64_t)(loc->nx + c.lt + c.rt) * (loc->ny + c.dn + c.up) * loc->nf;
+   const int64_t numExt = pvgpu::to_loc(*loc).numExt();
    if (total > 0x7fffffff || numExt > 0x7fffffff) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   c.numNeurons = (int)numNeurons;
    c.total = (int)total;
-   c.numExt = (int)numExt;
+   c.map = pvgpu::row_map(pvgpu::to_loc(*loc), 1);
    cudaStream_t s = pvgpu::as_stream(stream);
    uint4 *r = reinterpret_cast<uint4 *>(rnd);
-   const int grid = grid_for(total);
+   const int grid = (int)((total + 255) / 256);
    if (method == 'a') lif_kernel<'a'><<<grid, 256, 0, s>>>(c, r, V, Vth, GE, GI, GIB, gsynHead, aExt);
    else if (method == 'b') lif_kernel<'b'><<<grid, 256, 0, s>>>(c, r, V, Vth, GE, GI, GIB, gsynHead, aExt);
    else lif_kernel<'o'><<<grid, 256, 0, s>>>(c, r, V, Vth, GE, GI, GIB, gsynHead, aExt);
