@@ -471,7 +471,7 @@ enum {
    PVGPU_LCA_BF16 = 1  /* tcgen05 BF16 GEMMs with FP32 accumulation, FP32 residual and V */
 };
 
-/* Allocates the solver's device state (V, activity, reconstruction partials, weight copies). */
+/* Allocates the solver's device state (V, activity, residual and reconstruction buffers, weight copies). */
 pvgpu_status pvgpu_lca_solver_create(const pvgpu_lca_solver_desc *desc, pvgpu_lca_solver **out);
 pvgpu_status pvgpu_lca_solver_destroy(pvgpu_lca_solver *s);
 /* w: device FP32 [v1Nf][nxp][nxp][inNf], the V1 -> error weights (already normalised). */

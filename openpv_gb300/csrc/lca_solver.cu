@@ -1546,9 +1546,8 @@ __global__ void pad_x_kernel(LcaGeom g, int C, int E, int rowsPad, int RP, const
 // (ColumnEnergyProbe.cpp:60-70 over L2NormProbe and L1NormLCAProbe / FirmThresholdCostFnLCAProbe)
 // -------------------------------------------------------------------------------------------
 // The residual comes from the padded residual of kernel R (zero border) when rpad is given,
-// else from x and the partial reconstructions of the FP32 form.
+// else (no timestep since the reset) it is x.
 __global__ void __launch_bounds__(256) energy_kernel(LcaGeom g, int C, const float *__restrict__ x,
-                                                     const float *__restrict__ partials,
                                                      const float *__restrict__ rpad, int padPerImage,
                                                      const float *__restrict__ V, double l2Coeff, int costKind,
                                                      double cp0, double cp1, double costCoeff,
@@ -1563,11 +1562,8 @@ __global__ void __launch_bounds__(256) energy_kernel(LcaGeom g, int C, const flo
          l2 += r * r;
       }
    } else {
-      const float *pb = partials + (size_t)b * g.MB * nPix;
       for (int i = threadIdx.x; i < nPix; i += 256) {
-         float rec = pb[i];
-         for (int m = 1; m < g.MB; m++) rec = __fadd_rn(rec, pb[(size_t)m * nPix + i]);
-         double r = (double)__fadd_rn(x[(size_t)b * nPix + i], -rec);
+         const double r = (double)x[(size_t)b * nPix + i];
          l2 += r * r;
       }
    }
@@ -1686,7 +1682,7 @@ __global__ void v_layout_kernel(LcaGeom g, const float *__restrict__ src, float 
 // The SIMT FP32 form lives in lca_solver_fp32.cu and shares LcaGeom through this hook.
 namespace pvgpu {
 pvgpu_status lca_fp32_step(int S, int P, int C, const LcaGeom &g, const float *x, const float *W32, const float *Wt32,
-                           float *partials, float *V, float *A32, cudaStream_t s, cudaEvent_t mid);
+                           float *D, float *rpad, float *V, float *A32, cudaStream_t s, cudaEvent_t mid);
 }
 
 // Images [img0, img0 + g.nb) of the batch as a batch of their own: the geometry and the tensor
@@ -1703,7 +1699,7 @@ struct pvgpu_lca_solver {
    LcaGeom g;
    int S, P, C, KP;
    int stepsRun;
-   float *V = nullptr, *partials = nullptr, *A32 = nullptr, *W32 = nullptr, *Wt32 = nullptr;
+   float *V = nullptr, *A32 = nullptr, *W32 = nullptr, *Wt32 = nullptr;
    float *rpad = nullptr;  // padded residual x - W^T a (kernel D -> kernel P)
    bf16 *A = nullptr, *Alo = nullptr, *W = nullptr, *Wlo = nullptr, *Wt = nullptr, *Wtlo = nullptr;
    int *err = nullptr;
@@ -1714,7 +1710,9 @@ struct pvgpu_lca_solver {
    float *bands = nullptr;  // kernel F's bands, two buffers (a step reads one and writes the other)
    float *xpad = nullptr;   // x in the padded layout (kernel F)
    size_t bandsPerBuf = 0;  // floats in one band buffer (sized for 128-feature tiles)
-   bool padValid = false;  // rpad holds the residual of the last step (BF16 form) rather than partials
+   float *D32 = nullptr;    // the FP32 form's A . W [nbatch * positions][KP]: its own, or the bands' memory
+   bool ownD32 = false;
+   bool padValid = false;  // rpad holds the residual of the last step
    bool weightsSet = false;
    // optional per-kernel timing: events before kernel R, between R and P, after P
    std::vector<cudaEvent_t> ev;
@@ -2141,7 +2139,7 @@ void free_solver(pvgpu_lca_solver *s) {
    if (s->capStream2) cudaStreamDestroy(s->capStream2);
    if (s->forkEv) cudaEventDestroy(s->forkEv);
    if (s->joinEv) cudaEventDestroy(s->joinEv);
-   void *ptrs[] = {s->V,   s->partials, s->rpad, s->A32, s->W32, s->Wt32,  s->A,
+   void *ptrs[] = {s->V,   s->ownD32 ? s->D32 : nullptr, s->rpad, s->A32, s->W32, s->Wt32,  s->A,
                    s->Alo, s->W,        s->Wlo,  s->Wt,  s->Wtlo, s->bands, s->xpad, s->err};
    for (void *p : ptrs)
       if (p) cudaFree(p);
@@ -2239,13 +2237,12 @@ extern "C" pvgpu_status pvgpu_lca_solver_create(const pvgpu_lca_solver_desc *d, 
    g.si = d->selfInteract ? 1.0f : 0.0f;
    g.simple = (vw == 0.0f && !(d->AMax < FLT_MAX) && vt > -FLT_MAX) ? 1 : 0;
    const size_t nState = (size_t)g.nb * Npos * g.F;
-   const size_t nPart = (size_t)g.nb * g.MB * d->inNx * d->inNy * C;
    const size_t nW = (size_t)g.F * KP;
    const int E = (P - S) / 2;
    const size_t nPad = (size_t)g.nb * (d->inNy + 2 * E) * (((d->inNx + 2 * E) * C + 3) & ~3);
    bool ok = cudaMalloc(&s->V, nState * 4) == cudaSuccess && cudaMalloc(&s->A32, nState * 4) == cudaSuccess &&
              cudaMalloc(&s->A, nState * 2) == cudaSuccess && cudaMalloc(&s->Alo, nState * 2) == cudaSuccess &&
-             cudaMalloc(&s->partials, nPart * 4) == cudaSuccess && cudaMalloc(&s->W, nW * 2) == cudaSuccess &&
+             cudaMalloc(&s->W, nW * 2) == cudaSuccess &&
              cudaMalloc(&s->Wlo, nW * 2) == cudaSuccess && cudaMalloc(&s->Wt, nW * 2) == cudaSuccess &&
              cudaMalloc(&s->Wtlo, nW * 2) == cudaSuccess && cudaMalloc(&s->W32, nW * 4) == cudaSuccess &&
              cudaMalloc(&s->Wt32, nW * 4) == cudaSuccess && cudaMalloc(&s->err, sizeof(int)) == cudaSuccess &&
@@ -2318,6 +2315,16 @@ extern "C" pvgpu_status pvgpu_lca_solver_create(const pvgpu_lca_solver_desc *d, 
          s->xpad = nullptr;
          std::memset(&s->fplan, 0, sizeof(s->fplan));
       }
+   }
+   // the FP32 form's reconstruction GEMM output lives in the bands, which hold nothing between runs,
+   // where they are large enough
+   const size_t nD = (size_t)g.nb * Npos * KP;
+   if (s->bands && 2 * s->bandsPerBuf >= nD) s->D32 = s->bands;
+   else if (cudaMalloc(&s->D32, nD * 4) == cudaSuccess) s->ownD32 = true;
+   else {
+      cudaGetLastError();
+      free_solver(s);
+      return PVGPU_ERR_OOM;
    }
    s->rplan = make_recon_plan(g, S, P, C, false, g_num_sms);
    s->rplanX3 = make_recon_plan(g, S, P, C, true, g_num_sms);
@@ -2407,7 +2414,7 @@ extern "C" pvgpu_status pvgpu_lca_solver_run(pvgpu_lca_solver *s, const float *x
       for (int t = 0; t < numSteps; t++) {
          const bool rec = s->profiling && s->evNext + 3 <= s->ev.size();
          if (rec) cudaEventRecord(s->ev[s->evNext], st);
-         pvgpu_status r = pvgpu::lca_fp32_step(s->S, s->P, s->C, s->g, x, s->W32, s->Wt32, s->partials, s->V, s->A32,
+         pvgpu_status r = pvgpu::lca_fp32_step(s->S, s->P, s->C, s->g, x, s->W32, s->Wt32, s->D32, s->rpad, s->V, s->A32,
                                                st, rec ? s->ev[s->evNext + 1] : nullptr);
          if (r != PVGPU_OK) return r;
          if (rec) {
@@ -2416,7 +2423,7 @@ extern "C" pvgpu_status pvgpu_lca_solver_run(pvgpu_lca_solver *s, const float *x
          }
       }
       s->stepsRun += numSteps;
-      if (numSteps > 0) s->padValid = false;
+      if (numSteps > 0) s->padValid = true;
       return PVGPU_OK;
    }
    if (precision != PVGPU_LCA_BF16) return PVGPU_ERR_BAD_ARG;
@@ -2476,7 +2483,7 @@ extern "C" pvgpu_status pvgpu_lca_solver_energy(pvgpu_lca_solver *s, const float
                                                 double costThresh, double costWidth, double costCoeff,
                                                 double *energy, void *stream) {
    if (!s || !x || !energy || (costKind != 1 && costKind != 2)) return PVGPU_ERR_BAD_ARG;
-   energy_kernel<<<s->g.nb, 256, 0, pvgpu::as_stream(stream)>>>(s->g, s->C, x, s->partials,
+   energy_kernel<<<s->g.nb, 256, 0, pvgpu::as_stream(stream)>>>(s->g, s->C, x,
                                                                 s->padValid ? s->rpad : nullptr, s->rplan.rowsPad * s->rplan.RP,
                                                                 s->V, l2Coeff, costKind, costThresh, costWidth,
                                                                 costCoeff, energy);
