@@ -207,17 +207,32 @@ def check(status, what):
 
 # ---- torch plumbing ---------------------------------------------------------------------
 
+# A call of one of the small layers takes the GPU 2 to 10 us, so what is done here per argument shows:
+# pointers and streams go through as plain integers (the declared argument types convert them), and the
+# current stream's handle is asked for without making a Stream object.
+
 def _ptr(t):
     if t is None:
         return None
     assert t.is_cuda and t.is_contiguous(), "device tensors must be contiguous CUDA tensors"
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_current_raw_stream = None
 
 
 def _stream(stream=None):
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    global _current_raw_stream
+    if _current_raw_stream is None:
+        import torch
+        raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.current_device
+        if raw is not None:
+            _current_raw_stream = lambda: raw(device())  # noqa: E731
+        else:
+            _current_raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    return _current_raw_stream()
 
 
 def conn_desc(pre, post, nxp, nyp, dt_factor=1.0):
@@ -226,10 +241,10 @@ def conn_desc(pre, post, nxp, nyp, dt_factor=1.0):
 
 def compact_active(a_ext, nbatch, num_ext, entries, num_active, scratch=None, stream=None):
     """entries: uint8/int64 tensor viewed as [nbatch][num_ext] {u32 index, f32 value}."""
-    import torch
-    need = lib().pvgpu_compact_scratch_bytes(nbatch, num_ext)
     if scratch is None:
-        scratch = torch.empty(max(need, 1), dtype=torch.uint8, device=a_ext.device)
+        import torch
+        scratch = torch.empty(max(lib().pvgpu_compact_scratch_bytes(nbatch, num_ext), 1), dtype=torch.uint8,
+                              device=a_ext.device)
     check(lib().pvgpu_compact_active(_ptr(a_ext), nbatch, num_ext, _ptr(entries), _ptr(num_active), _ptr(scratch),
                                      scratch.numel() * scratch.element_size(), _stream(stream)), "compact_active")
 
