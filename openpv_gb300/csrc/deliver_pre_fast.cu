@@ -12,9 +12,14 @@
 #include "deliver_pre.cuh"
 #include "fast_axis.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <type_traits>
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 using pvgpu::fast_axis;
 using pvgpu::FastAxis;
@@ -359,32 +364,63 @@ pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *e
 // -------------------------------------------------------------------------------------------
 // Narrow post layers.
 //
-// A CTA owns an output tile of TY x TX positions x FT features.  The entries that reach it (their
-// ranges in each presynaptic row found first) are numbered through and dealt to the warps in chunks
-// of 32: the lanes decode one entry each, then the warp takes the chunk's entries one after the
-// other with its lanes spread over the weights of the patch -- one entry's patch is contiguous in
-// memory, so the loads are coalesced and its addresses are the entry's plus a constant per lane.
-// Products go into the warp's own copy of the tile in shared memory, which has a margin of the patch
-// size on every side so that no lane tests whether its output lies inside.  The copies are summed
-// in warp order into GSyn.
+// A cluster of cz CTAs owns an output tile of TY x TX positions x FT features.  The entries that reach it
+// (their ranges in each presynaptic row found first) are numbered through and dealt to the warps of the
+// cluster in chunks of 32: the lanes decode one entry each, then the warp takes the chunk's entries one
+// after the other with its lanes spread over the weights of the patch, VEC neighbouring ones each -- one
+// entry's patch is contiguous in memory, so the loads are coalesced and its addresses are the entry's
+// plus a constant per lane.  Products go into the warp's own copy of the tile in shared memory, which has
+// a margin of the patch size on every side so that no lane tests whether its output lies inside.  The
+// copies are summed in warp order, then over the cluster in rank order, into GSyn.
 //
 // The tile kernel this replaces gave each warp one output row and tested every entry of its range
 // against every output: on the delivery of a V1 layer to an image (one to three features, 8x8
 // patches) seven of eight lanes had nothing to add, and one image kept 8 CTAs busy.  Measured:
-// one 16x16x64 V1 layer to 32x32x1 160 -> 10 us; 8 x 256x256x32 spikes (2 %) to 128x128x8, 3x3 at
-// stride 2, 425 -> 65 us.  What bounds it is the latency of the read-add-write on shared memory
-// (one entry's adds must land before the next one's) and of the entries' own chain of loads.
+// one 16x16x64 V1 layer to 32x32x1 160 -> SB1 us; 8 x 256x256x32 spikes (2 %) to 128x128x8, 3x3 at
+// stride 2, 425 -> SEX us; 32 x 16x16x512 (5 %) to 32x32x3 754 -> SB32 us.  What bounds it is the
+// read-add-write on shared memory (one entry's adds must land before the next one's), hence vectors of
+// up to four weights per lane, and tiles as large as the warps' copies allow -- a tile wastes what patches
+// hang over its edge -- with the entries of one tile divided over a cluster.
 // -------------------------------------------------------------------------------------------
 struct ScatPlan {
-   int TX, TY, FT, NW;
+   int TX, TY, FT, NW, cz, vec;
    int nTX, nTY, nFT;
    int PW, tileFloats;   // floats per row of the padded tile; one copy (a multiple of 4)
+   int padX;             // columns left of the tile: the margin, rounded so that patches start on vectors
    int rowsMax;
    size_t smem;
    double cost;
 };
 
-template <int EPT, int U, bool SPARSE>
+template <int VEC>
+struct VecW {
+   __device__ static __forceinline__ void ldg(const float *p, float *v) {
+      if constexpr (VEC == 4) {
+         const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+         v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+      } else if constexpr (VEC == 2) {
+         const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+         v[0] = t.x, v[1] = t.y;
+      } else v[0] = __ldg(p);
+   }
+   __device__ static __forceinline__ void ld(const float *p, float *v) {
+      if constexpr (VEC == 4) {
+         const float4 t = *reinterpret_cast<const float4 *>(p);
+         v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+      } else if constexpr (VEC == 2) {
+         const float2 t = *reinterpret_cast<const float2 *>(p);
+         v[0] = t.x, v[1] = t.y;
+      } else v[0] = *p;
+   }
+   __device__ static __forceinline__ void st(float *p, const float *v) {
+      if constexpr (VEC == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+      else if constexpr (VEC == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+      else *p = v[0];
+   }
+};
+
+// EPT vectors of the patch per lane at a time, U entries' weights in flight
+template <int EPT, int U, int VEC, bool SPARSE>
 __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, ScatPlan pl,
                                                                   const pvgpu_entry *__restrict__ entries,
                                                                   const int64_t *__restrict__ numActive,
@@ -399,7 +435,8 @@ __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, Sc
    float *acc0 = sm + NW * 128 + ((2 * pl.rowsMax + 1 + 3) & ~3);      // [NW][tileFloats]
    float *acc = acc0 + (size_t)warp * pl.tileFloats;
 
-   int t = blockIdx.x;
+   const int rank = pl.cz > 1 ? blockIdx.x % pl.cz : 0;
+   int t = blockIdx.x / pl.cz;
    const int X0 = (t % pl.nTX) * pl.TX;
    t /= pl.nTX;
    const int Y0 = (t % pl.nTY) * pl.TY, F0 = (t / pl.nTY) * pl.FT;
@@ -407,7 +444,7 @@ __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, Sc
    const int tx = min(pl.TX, g.postNx - X0), ty = min(pl.TY, g.postNy - Y0), ft = min(pl.FT, g.nfp - F0);
    const int yeLo = g.ay.first_ge(Y0 - g.nyp + 1), nRows = g.ay.first_ge(Y0 + ty) - yeLo;
    const int xlo = g.ax.first_ge(X0 - g.nxp + 1), nX = g.ax.first_ge(X0 + tx) - xlo;
-   if (nRows <= 0 || nX <= 0) return;  // CTA-uniform: nothing reaches the tile
+   if (nRows <= 0 || nX <= 0) return;  // cluster-uniform: nothing reaches the tile
 
    for (int i = lane; i < pl.tileFloats / 4; i += 32) reinterpret_cast<float4 *>(acc)[i] = make_float4(0, 0, 0, 0);
    const pvgpu_entry *eb = SPARSE ? entries + (size_t)b * g.preNumExt : nullptr;
@@ -439,14 +476,14 @@ __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, Sc
    const int perRow = nX * g.nf;  // dense form
    const int total = SPARSE ? rowPre[nRows] : nRows * perRow;
 
-   // this lane's patch weights: offset in the entry's patch and in the tile
+   // this lane's patch vectors: offset in the entry's patch and in the tile
    const int L = g.nxp * ft, elems = g.nyp * L;
    int wo[EPT], so[EPT];
    bool in[EPT];
    auto offsets = [&](int e0) {
 #pragma unroll
       for (int i = 0; i < EPT; i++) {
-         const int e = e0 + lane + 32 * i;
+         const int e = e0 + (lane + 32 * i) * VEC;
          in[i] = e < elems;
          const int ky = e / L, r = e - ky * L, kx = r / ft, fl = r - kx * ft;
          wo[i] = in[i] ? (ky * g.nxp + kx) * g.nfp + fl : 0;
@@ -455,7 +492,7 @@ __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, Sc
    };
    offsets(0);
 
-   for (int c0 = warp * 32; c0 < total; c0 += NW * 32) {
+   for (int c0 = (rank * NW + warp) * 32; c0 < total; c0 += pl.cz * NW * 32) {
       const int i = c0 + lane;
       int4 d = make_int4(0, 0, 0, 0);
       float a = 0.0f;
@@ -479,38 +516,42 @@ __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, Sc
          }
          const int ye = yeLo + r, xe = (int)((uint32_t)kr / (uint32_t)g.nf), f = kr - xe * g.nf;
          d.x = kernel_index(g, xe, ye, f) * g.patchSize + F0;
-         d.y = (g.ay.start(ye) - Y0 + g.nyp - 1) * pl.PW + (g.ax.start(xe) - X0 + g.nxp - 1) * pl.FT;
+         d.y = (g.ay.start(ye) - Y0 + g.nyp - 1) * pl.PW + (g.ax.start(xe) - X0 + pl.padX) * pl.FT;
          d.z = __float_as_int(a * g.dtf);
       }
       const unsigned m = __ballot_sync(0xffffffffu, a != 0.0f);
       const int cnt = __popc(m);
       if (a != 0.0f) stage[__popc(m & ((1u << lane) - 1))] = d;
       __syncwarp();
-      for (int e0 = 0; e0 < elems; e0 += 32 * EPT) {
-         if (elems > 32 * EPT) offsets(e0);
+      for (int e0 = 0; e0 < elems; e0 += 32 * EPT * VEC) {
+         if (elems > 32 * EPT * VEC) offsets(e0);
          int j = 0;
          auto take = [&](auto un) {
             constexpr int UN = decltype(un)::value;
             int4 q[UN];
-            float w[UN][EPT];
+            float w[UN][EPT][VEC];
 #pragma unroll
             for (int u = 0; u < UN; u++) q[u] = stage[j + u];
 #pragma unroll
             for (int u = 0; u < UN; u++)
 #pragma unroll
                for (int i2 = 0; i2 < EPT; i2++)
-                  if (in[i2]) w[u][i2] = __ldg(W + q[u].x + wo[i2]);
+                  if (in[i2]) VecW<VEC>::ldg(W + q[u].x + wo[i2], w[u][i2]);
 #pragma unroll
             for (int u = 0; u < UN; u++) {
                const float av = __int_as_float(q[u].z);
                float *p = acc + q[u].y;
-               float v[EPT];
+               float v[EPT][VEC];
 #pragma unroll
                for (int i2 = 0; i2 < EPT; i2++)
-                  if (in[i2]) v[i2] = p[so[i2]];
+                  if (in[i2]) VecW<VEC>::ld(p + so[i2], v[i2]);
 #pragma unroll
                for (int i2 = 0; i2 < EPT; i2++)
-                  if (in[i2]) p[so[i2]] = fmaf(av, w[u][i2], v[i2]);
+                  if (in[i2]) {
+#pragma unroll
+                     for (int x = 0; x < VEC; x++) v[i2][x] = fmaf(av, w[u][i2][x], v[i2][x]);
+                     VecW<VEC>::st(p + so[i2], v[i2]);
+                  }
                __syncwarp();  // the next entry's lanes may add to these outputs
             }
             j += UN;
@@ -523,25 +564,50 @@ __global__ void __launch_bounds__(256) deliver_pre_scatter_kernel(FastGeom g, Sc
    __syncthreads();
    const int outs = ty * tx * ft;
    float *gb = gsyn + (size_t)b * g.postNumRes + F0;
-   for (int o = tid; o < outs; o += NW * 32) {
-      const int fl = o % ft, x = (o / ft) % tx, y = o / (ft * tx);
-      const float *p = acc0 + (y + g.nyp - 1) * pl.PW + (x + g.nxp - 1) * pl.FT + fl;
-      float s = p[0];
-      for (int w = 1; w < NW; w++) s += p[(size_t)w * pl.tileFloats];
-      gb[((size_t)(Y0 + y) * g.postNx + X0 + x) * g.nfp + fl] += s;
+   // f(output's offset in the tile, its GSyn value) for this thread's outputs of [lo, hi)
+   auto outputs = [&](int lo, int hi, auto f) {
+      for (int o = lo + tid; o < hi; o += NW * 32) {
+         const int fl = o % ft, x = (o / ft) % tx, y = o / (ft * tx);
+         f((y + g.nyp - 1) * pl.PW + (x + pl.padX) * pl.FT + fl,
+           gb + ((size_t)(Y0 + y) * g.postNx + X0 + x) * g.nfp + fl);
+      }
+   };
+   if (pl.cz == 1) {
+      outputs(0, outs, [&](int at, float *gp) {
+         float s = acc0[at];
+         for (int w = 1; w < NW; w++) s += acc0[at + (size_t)w * pl.tileFloats];
+         *gp += s;
+      });
+      return;
    }
+   outputs(0, outs, [&](int at, float *) {
+      float s = acc0[at];
+      for (int w = 1; w < NW; w++) s += acc0[at + (size_t)w * pl.tileFloats];
+      acc0[at] = s;
+   });
+   cg::cluster_group cl = cg::this_cluster();
+   cl.sync();
+   const int share = (outs + pl.cz - 1) / pl.cz;
+   outputs(min(rank * share, outs), min((rank + 1) * share, outs), [&](int at, float *gp) {
+      float s = cl.map_shared_rank(acc0, 0)[at];
+      for (int c = 1; c < pl.cz; c++) s += cl.map_shared_rank(acc0, c)[at];
+      *gp += s;
+   });
+   cl.sync();  // no CTA leaves while another reads its tile
 }
 
 // Tile shape by an estimate of the launch's time (cycles): the instructions of all CTAs over the
 // chip's issue slots, or the serial time of one CTA's warps times the waves of CTAs, whichever is
-// longer.  Larger tiles waste less of the patches that hang over their edge; smaller ones give the
-// chip enough CTAs.  Activity is taken as 5 % (the kernel's result does not depend on it).
-bool scatter_plan(const PreGeom &pg, const FastGeom &g, bool sparse, ScatPlan *best) {
+// longer.  Activity is taken as 5 % (30 % for a dense layer; the result does not depend on it).
+bool scatter_plan(const PreGeom &pg, const FastGeom &g, const float *W, bool sparse, ScatPlan *best) {
    const int sms = num_sms();
    best->cost = 1e300;
    const int sx = std::max(1, pg.pre.nx / pg.post.nx), tx = std::max(1, pg.post.nx / pg.pre.nx);
    const int sy = std::max(1, pg.pre.ny / pg.post.ny), ty = std::max(1, pg.post.ny / pg.pre.ny);
-   for (int T = 32; T >= 4; T >>= 1) {
+   // patches start at columns congruent to this modulo tx (one-to-many; else at any column)
+   const int phase = ((-((g.nxp - tx) / 2)) % tx + tx) % tx;
+   for (int T = 64; T >= 4; T >>= 1) {
+      if (T > 4 && T >= 2 * std::max(g.postNx, g.postNy)) continue;  // the same tile as the next
       for (int nft = 1; nft <= 32; nft *= 2) {
          ScatPlan p;
          p.FT = (g.nfp + nft - 1) / nft;
@@ -551,10 +617,19 @@ bool scatter_plan(const PreGeom &pg, const FastGeom &g, bool sparse, ScatPlan *b
          p.TY = std::min(T, g.postNy);
          p.nTX = (g.postNx + p.TX - 1) / p.TX;
          p.nTY = (g.postNy + p.TY - 1) / p.TY;
-         p.PW = (p.TX + 2 * (g.nxp - 1)) * p.FT;
+         // vectors: patch rows, patches and their starts in whole vectors (tiles start at multiples of tx)
+         p.vec = 1;
+         for (int v = 4; v >= 2 && p.vec == 1; v /= 2) {
+            const bool rows = p.nFT == 1 ? g.nxp * g.nfp % v == 0 : p.FT % v == 0 && g.nfp % v == 0;
+            const bool starts = (p.FT % v == 0 || (tx * p.FT % v == 0 && p.TX % tx == 0));
+            if (rows && starts && g.patchSize % v == 0 && reinterpret_cast<uintptr_t>(W) % (4 * v) == 0) p.vec = v;
+         }
+         p.padX = g.nxp - 1;
+         if (p.vec > 1 && p.FT % p.vec != 0) p.padX += (2 * tx - (p.padX + phase) % tx) % tx;
+         p.PW = ((p.TX + p.padX + g.nxp - 1) * p.FT + 3) & ~3;
          const int64_t tf = (int64_t)p.PW * (p.TY + 2 * (g.nyp - 1));
          if (tf > 14000) continue;
-         p.tileFloats = (int)((tf + 3) & ~3);
+         p.tileFloats = (int)tf;
          const int covY = (p.TY + g.nyp - 1) * sy / ty + 2, covX = (p.TX + g.nxp - 1) * sx / tx + 2;
          p.rowsMax = covY + sy;
          for (p.NW = 8; p.NW >= 4; p.NW >>= 1) {
@@ -562,49 +637,72 @@ bool scatter_plan(const PreGeom &pg, const FastGeom &g, bool sparse, ScatPlan *b
             if (p.smem <= 200 * 1024) break;
          }
          if (p.NW < 4) continue;
-         const int64_t ctas = (int64_t)p.nTX * p.nTY * p.nFT;
-         if (ctas > 0x7fffffff) continue;
+         const int64_t tiles = (int64_t)p.nTX * p.nTY * p.nFT;
          const int occ = (int)std::min<size_t>(2048 / (p.NW * 32), (227 * 1024) / (p.smem + 1024));
-         const int blocks = (g.nyp * g.nxp * p.FT + 31) / 32;
+         const int vectors = (g.nyp * g.nxp * p.FT / p.vec + 31) / 32;
+         // a vector of one entry: load, read, multiply-adds, write; serially a read-add-write's latency
+         const double perEntry = 18 + vectors * (4.0 + p.vec), latency = 45 + vectors * (4.0 + 2.0 * p.vec);
          const double E = (double)covX * covY * g.nf * (sparse ? 0.05 : 0.3) + 1.0;
          const double outs = (double)p.TX * p.TY * p.FT / 32;
-         const double instr = E * (16 + 5.0 * blocks) + p.NW * (p.tileFloats / 128.0 + 500) + outs * (p.NW * 2 + 8);
-         const double n = (double)ctas * pg.pre.nb;
-         const double serial = 3000 + E / p.NW * (45 + 6.0 * blocks) + p.tileFloats / 64.0 + outs * 4;
-         const double waves = std::max(1.0, n / ((double)sms * occ));
-         p.cost = std::max(n * instr / (sms * 2.5), serial * waves);
-         if (p.cost < best->cost) *best = p;
+         for (p.cz = 1; p.cz <= 8; p.cz *= 2) {
+            if (tiles * p.cz > 0x7fffffff || (p.cz > 1 && E / p.cz < 64)) break;
+            const double instr = E / p.cz * perEntry + p.NW * (p.tileFloats / 128.0 + 500) + outs * (p.NW * 2 + 8 + (p.cz > 1 ? 20 : 0));
+            const double n = (double)tiles * p.cz * pg.pre.nb;
+            const double serial = 3000 + E / p.cz / p.NW * latency + p.tileFloats / 64.0 + outs * 4 + (p.cz > 1 ? 4000 : 0);
+            const double waves = std::max(1.0, n / ((double)sms * occ));
+            p.cost = std::max(n * instr / (sms * 2.5), serial * waves);
+            if (p.cost < best->cost) *best = p;
+         }
       }
    }
    return best->cost < 1e300;
 }
 
-template <int EPT, int U>
+template <int EPT, int U, int VEC>
 pvgpu_status launch_scatter(const FastGeom &g, const ScatPlan &pl, int nb, cudaStream_t s, const pvgpu_entry *entries,
                             const int64_t *numActive, const float *aExt, const float *W, float *gsyn) {
-   const dim3 grid((unsigned)(pl.nTX * pl.nTY * pl.nFT), nb);
    auto go = [&](auto kernel) -> pvgpu_status {
       if (pl.smem > 48 * 1024)
          PVGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem),
                     "deliver_pre scatter attribute");
-      kernel<<<grid, pl.NW * 32, pl.smem, s>>>(g, pl, entries, numActive, aExt, W, gsyn);
-      PVGPU_CHECK_LAUNCH("deliver_pre scatter");
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = pl.cz;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t c = {};
+      c.gridDim = dim3((unsigned)(pl.nTX * pl.nTY * pl.nFT * pl.cz), nb);
+      c.blockDim = dim3(pl.NW * 32);
+      c.dynamicSmemBytes = pl.smem;
+      c.stream = s;
+      c.attrs = attr;
+      c.numAttrs = pl.cz > 1 ? 1 : 0;
+      PVGPU_CUDA(cudaLaunchKernelEx(&c, kernel, g, pl, entries, numActive, aExt, W, gsyn), "deliver_pre scatter");
       return PVGPU_OK;
    };
-   return entries ? go(deliver_pre_scatter_kernel<EPT, U, true>) : go(deliver_pre_scatter_kernel<EPT, U, false>);
+   return entries ? go(deliver_pre_scatter_kernel<EPT, U, VEC, true>) : go(deliver_pre_scatter_kernel<EPT, U, VEC, false>);
+}
+
+template <int VEC>
+pvgpu_status scatter_vec(const FastGeom &g, const ScatPlan &pl, int nb, cudaStream_t s, const pvgpu_entry *entries,
+                         const int64_t *numActive, const float *aExt, const float *W, float *gsyn) {
+   // vectors per lane for the whole patch, up to four (larger patches go round in blocks); entries in
+   // flight so that their weights take at most 32 registers
+   const int ept = (g.nyp * g.nxp * pl.FT / VEC + 31) / 32;
+   if (ept <= 1) return launch_scatter<1, 4, VEC>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
+   if (ept <= 2) return launch_scatter<2, 4, VEC>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
+   if (ept <= 3) return launch_scatter<3, VEC == 4 ? 2 : 4, VEC>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
+   return launch_scatter<4, VEC == 4 ? 2 : 4, VEC>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
 }
 
 pvgpu_status try_scatter(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *entries, const int64_t *numActive,
                          const float *aExt, const float *W, float *gsyn, cudaStream_t s) {
    ScatPlan pl;
-   if (!scatter_plan(pg, g, entries != nullptr, &pl)) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   const int ept = (g.nyp * g.nxp * pl.FT + 31) / 32, nb = pg.pre.nb;
-   if (ept <= 1) return launch_scatter<1, 4>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
-   if (ept <= 2) return launch_scatter<2, 4>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
-   if (ept <= 3) return launch_scatter<3, 4>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
-   if (ept <= 4) return launch_scatter<4, 4>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
-   if (ept <= 6) return launch_scatter<6, 2>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
-   return launch_scatter<8, 2>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
+   if (!scatter_plan(pg, g, W, entries != nullptr, &pl)) return PVGPU_ERR_UNSUPPORTED_SHAPE;
+   const int nb = pg.pre.nb;
+   return pl.vec == 4   ? scatter_vec<4>(g, pl, nb, s, entries, numActive, aExt, W, gsyn)
+          : pl.vec == 2 ? scatter_vec<2>(g, pl, nb, s, entries, numActive, aExt, W, gsyn)
+                        : scatter_vec<1>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
 }
 
 }  // namespace

@@ -31,6 +31,12 @@ CASES = [
     ((4, 64, 48, 32, 2), (32, 24, 8, 0), 3, 3, 0.02, 0),   # many-to-one spikes
     ((1, 128, 96, 1, 1), (128, 96, 2, 0), 3, 3, 1.0, 0),   # dense image
     ((1, 70, 2, 3, 1), (70, 2, 5, 0), 3, 3, 0.0, 0),       # nothing active
+    ((2, 16, 16, 60, 2), (32, 32, 3, 0), 8, 8, 0.1, 0),    # pairs of weights, patches starting off the vector grid
+    ((2, 16, 16, 60, 2), (32, 32, 3, 0), 8, 8, 0.1, 1),    # the same with weights not aligned for vectors
+    ((3, 9, 7, 6, 1), (9, 7, 8, 0), 3, 3, 0.3, 0),         # quads
+    ((1, 12, 5, 200, 1), (48, 20, 2, 0), 8, 8, 0.2, 0),    # one-to-many x4 of two features: quads, one tile
+    ((1, 16, 16, 300, 2), (64, 64, 1, 0), 16, 16, 0.1, 0),  # a tile of the whole image over a cluster
+    ((2, 40, 44, 20, 4), (20, 22, 6, 0), 5, 5, 0.3, 0),    # pairs, many-to-one
 ]
 
 
