@@ -67,26 +67,50 @@ __device__ __forceinline__ int kernel_index(const FastGeom &g, int xe, int ye, i
 
 // lower_bound of `keys` extended indices in the ascending list e[0, n), eight lanes to a key: each
 // round cuts the range to an eighth, so a list of 40,000 entries takes five dependent loads instead
-// of sixteen.  put(t, position) is called by one lane for each key t.
+// of sixteen; and each group of lanes searches for four keys at once, so that those loads overlap (one
+// key at a time cost a CTA that visits 36 rows 15 round trips to L2).  put(t, position) is called by one
+// lane for each key t.
 template <typename Key, typename Put>
 __device__ __forceinline__ void search_keys(const pvgpu_entry *e, int n, int keys, Key key, Put put) {
+   constexpr int KP = 4;
    const int lane = threadIdx.x & 31, l = lane & 7, groups = blockDim.x >> 3;
    const unsigned gmask = 0xffu << (lane & 24);
-   for (int t0 = 0; t0 < keys; t0 += groups) {
-      const int t = t0 + (threadIdx.x >> 3);
-      const bool on = t < keys;
-      const int64_t k = on ? key(t) : 0;
-      int lo = 0, hi = on ? n : 0;
-      while (__any_sync(0xffffffffu, lo < hi)) {
-         const int q = (hi - lo + 7) >> 3, p = lo + q * (l + 1) - 1;
-         const bool less = lo < hi && p < hi && (int64_t)e[p].index < k;
-         const int cnt = __popc(__ballot_sync(0xffffffffu, less) & gmask);
-         if (lo < hi) {
-            hi = min(hi, lo + q * (cnt + 1) - 1);
-            lo += q * cnt;
+   for (int t0 = 0; t0 < keys; t0 += groups * KP) {
+      int64_t k[KP];
+      int lo[KP], hi[KP];
+#pragma unroll
+      for (int i = 0; i < KP; i++) {
+         const int t = t0 + i * groups + (threadIdx.x >> 3);
+         k[i] = t < keys ? key(t) : 0;
+         lo[i] = 0;
+         hi[i] = t < keys ? n : 0;
+      }
+      for (;;) {
+         bool open = false;
+         uint32_t at[KP];
+#pragma unroll
+         for (int i = 0; i < KP; i++) {
+            const int q = (hi[i] - lo[i] + 7) >> 3, p = lo[i] + q * (l + 1) - 1;
+            open = open || lo[i] < hi[i];
+            at[i] = lo[i] < hi[i] && p < hi[i] ? e[p].index : 0xffffffffu;
+         }
+         if (!__any_sync(0xffffffffu, open)) break;
+#pragma unroll
+         for (int i = 0; i < KP; i++) {
+            const int q = (hi[i] - lo[i] + 7) >> 3, p = lo[i] + q * (l + 1) - 1;
+            const bool less = lo[i] < hi[i] && p < hi[i] && (int64_t)at[i] < k[i];
+            const int cnt = __popc(__ballot_sync(0xffffffffu, less) & gmask);
+            if (lo[i] < hi[i]) {
+               hi[i] = min(hi[i], lo[i] + q * (cnt + 1) - 1);
+               lo[i] += q * cnt;
+            }
          }
       }
-      if (on && l == 0) put(t, lo);
+#pragma unroll
+      for (int i = 0; i < KP; i++) {
+         const int t = t0 + i * groups + (threadIdx.x >> 3);
+         if (t < keys && l == 0) put(t, lo[i]);
+      }
    }
 }
 
@@ -627,6 +651,9 @@ bool scatter_plan(const PreGeom &pg, const FastGeom &g, const float *W, bool spa
          p.padX = g.nxp - 1;
          if (p.vec > 1 && p.FT % p.vec != 0) p.padX += (2 * tx - (p.padX + phase) % tx) % tx;
          p.PW = ((p.TX + p.padX + g.nxp - 1) * p.FT + 3) & ~3;
+         // a patch's rows, of L values, in neighbouring banks: the pitch is L or -L modulo the 32 banks
+         if (const int L = (g.nxp * p.FT + 3) & 31 & ~3)
+            while (p.PW % 32 != L && p.PW % 32 != 32 - L) p.PW += 4;
          const int64_t tf = (int64_t)p.PW * (p.TY + 2 * (g.nyp - 1));
          if (tf > 14000) continue;
          p.tileFloats = (int)tf;
