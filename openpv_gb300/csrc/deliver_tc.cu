@@ -25,9 +25,9 @@
 // lo rows, NT x 32 TF32 each, pre-split in the workspace, 128-byte swizzle) stream through a
 // ring, each used by the R rows of a unit.
 //
-// MMA shape.  One tcgen05.mma costs about 117 cycles for N <= 128 and 171 for N = 256 (TF32,
-// M = 128, same accumulator), against 32 for N = 64 at the tensor pipe's peak, and switching
-// accumulators between consecutive MMAs costs more still.  So the hi and lo weight tiles are
+// MMA shape.  Back to back (TF32, M = 128), a tcgen05.mma of N = 256 takes 128 cycles, of N = 128 64 and
+// of N = 64 48 to 57 (its operands' 6 KB stream at 128 B per cycle), whatever the row it starts at;
+// switching accumulators at every MMA makes a pair 144 instead of 113.  So the hi and lo weight tiles are
 // one N = 2*NT operand: per K step, MMA 1 = A_hi x [W_hi; W_lo] (N = 2*NT) and MMA 2 =
 // A_lo x W_hi (N = NT) into the same accumulator (columns n: W_hi parts, NT + n: A_hi x W_lo),
 // two MMAs where three N = NT products would take three; the dropped A_lo x W_lo is below 2^-22
@@ -95,7 +95,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
 
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    const uint32_t bBytes = (uint32_t)g.NT * 128;  // one TF32 weight tile (NT rows x 32)
-   const int groupsPerUnit = g.nFC * g.KY;
    const int rowsPerFC = g.R + g.KY - 1;
 
    if (tid == 0) {
@@ -126,6 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
    const uint32_t tmem = tmemBase;
 
    auto wait_or_abort = [&](uint64_t *bar, uint32_t parity) {
+      if (mbar_try_wait(bar, parity)) return true;
       if (abortFlag) return false;
       if (mbar_wait(bar, parity)) return true;
       abortFlag = 1;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
    };
    // warp-uniform wait: every lane observes the phase; the warp goes on only if all of them did
    auto warp_wait = [&](uint64_t *bar, uint32_t parity) {
-      const bool mine = !abortFlag && mbar_wait(bar, parity);
+      const bool mine = mbar_try_wait(bar, parity) || (!abortFlag && mbar_wait(bar, parity));
       const bool all = __all_sync(0xffffffffu, mine) != 0;
       if (!all && lane == 0) abortFlag = 1;
       return all;
@@ -196,83 +196,115 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
       }
    } else if (warp == 1) {
       // ================================ MMA issuer ================================
-      if (lane == 0) {
-         const uint32_t idesc = idesc_tf32(128, 2 * g.NT), idescHi = idesc_tf32(128, g.NT);
-         // Descriptors are built once; an operand at byte offset o from its base is the base
-         // descriptor plus o >> 4 (the start-address field, which cannot carry: shared-memory
-         // addresses are below 2^18).
-         const uint64_t aD0 = sdesc_noswizzle(smem_u32(smem), kColA, 128);
-         const uint64_t bD0 = sdesc_sw128(smem_u32(smem + g.offB));
-         constexpr uint64_t kLoA = kHalfA >> 4, kStepA = (2 * kColA) >> 4;
-         uint32_t cbase = 0, cb = 0, cc = 0;  // split rows, weight tiles, chains so far
-         int slotBase = 0;                    // cbase % NS
-         int d = 0;                           // cb % NB
-         uint32_t bPar = 0;                   // (cb / NB) & 1
-         bool ok = true;
-         for (int u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
-            int grp = 0;
-            uint32_t tacc = 0;
-            for (int fc = 0; fc < g.nFC && ok; fc++) {
-               for (int ky = 0; ky < g.KY && ok; ky++, grp++) {
-                  const bool chainStart = grp % g.groupsPerChain == 0;
-                  if (chainStart) {
-                     const int buf = cc & 1;
-                     if (cc >= 2 && !(ok = wait_or_abort(&chainEmpty[buf], ((cc >> 1) - 1) & 1))) break;
-                     tc_fence_after();  // the epilogue's TMEM reads of this buffer precede the MMAs
-                     tacc = tmem + (uint32_t)(buf * 2 * NCH * 32);
-                  }
-                  // source rows ky .. ky+R-1 of this chunk must be split
-                  for (int j = ky == 0 ? 0 : ky + g.R - 1; j < ky + g.R && ok; j++) {
-                     const uint32_t c = cbase + j;
-                     ok = wait_or_abort(&aReady[c % g.NS], (c / g.NS) & 1);
-                  }
-                  if (!ok) break;
-                  // operands written by TMA or by proxy-fenced stores need no tcgen05 fence
-                  const int slotKy = (slotBase + ky) % g.NS;
-                  for (int kx = 0; kx < g.KX && ok; kx++) {
-                     if (!(ok = wait_or_abort(&bFull[d], bPar))) break;
-                     const uint64_t bd = bD0 + (uint64_t)((d * 2 * bBytes) >> 4);
-                     const uint32_t acc0 = fresh0(chainStart && kx == 0);
-                     uint64_t adr[R];
+      const uint32_t idesc = idesc_tf32(128, 2 * g.NT), idescHi = idesc_tf32(128, g.NT);
+      // Descriptors are built once; an operand at byte offset o from its base is the base
+      // descriptor plus o >> 4 (the start-address field, which cannot carry: shared-memory
+      // addresses are below 2^18).
+      const uint64_t aD0 = sdesc_noswizzle(smem_u32(smem), kColA, 128);
+      const uint64_t bD0 = sdesc_sw128(smem_u32(smem + g.offB));
+      constexpr uint64_t kLoA = kHalfA >> 4, kStepA = (2 * kColA) >> 4;
+      // The tensor pipe holds little beyond the MMA it runs, so whatever this warp does between two
+      // MMAs shows: with operands that never wait, the pair of a K step takes 113 cycles, and a probe
+      // of a barrier, a flag read and a commit per weight tile add 28 to each of its eight pairs
+      // (R = 2).  So the whole warp walks the units and one elected lane issues (operands stay in
+      // uniform registers: 28 -> 21), the next tile's barrier is probed in the middle of a tile's
+      // MMAs, positions advance by additions, and the abort flag is read only where a wait does not
+      // find its phase.  The 128x128x256 -> 64 delivery with 7x7 patches, batch 16: 2.09 -> 1.72 ms
+      // (0.62 -> 0.75 of the pairs' rate).  Tried: core matrices of every 16th position, so that a
+      // shift moves by whole 128-byte lines (the MMA rate does not depend on it; four weight tiles
+      // instead of six: 2.27); one barrier for two or three weight tiles (1.81); the probe after the
+      // first or the last MMAs (1.72); no copies of weights at all (2.07 before, 1.77 with lane 0
+      // issuing: the copies are not what the MMAs wait for).
+      const uint64_t stepB = (2 * bBytes) >> 4;
+      uint32_t cc = 0;      // chains so far
+      int slotA = 0;        // slot and phase of split row ky (the next one to lose its last use)
+      uint32_t parA = 0;
+      int d = 0;            // slot and phase of the next weight tile
+      uint32_t parB = 0;
+      uint64_t bd = bD0;
+      bool bSeen = false;   // the next weight tile's barrier was found complete
+      bool ok = true;
+      // split row `ahead` after slotA
+      auto row_ready = [&](int ahead) {
+         int sl = slotA + ahead;
+         uint32_t par = parA;
+         if (sl >= g.NS) {
+            sl -= g.NS;
+            par ^= 1u;
+         }
+         return warp_wait(&aReady[sl], par);
+      };
+      auto next_row = [&] {
+         if (++slotA == g.NS) {
+            slotA = 0;
+            parA ^= 1u;
+         }
+      };
+      for (int u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+         int chainLeft = 0;  // patch rows left in the open chain
+         uint32_t tacc = 0;
+         for (int fc = 0; fc < g.nFC && ok; fc++) {
+            for (int ky = 0; ky < g.KY && ok; ky++) {
+               const bool chainStart = chainLeft == 0;
+               if (chainStart) {
+                  chainLeft = g.groupsPerChain;
+                  const int buf = cc & 1;
+                  if (cc >= 2 && !(ok = warp_wait(&chainEmpty[buf], ((cc >> 1) - 1) & 1))) break;
+                  tc_fence_after();  // the epilogue's TMEM reads of this buffer precede the MMAs
+                  tacc = tmem + (uint32_t)(buf * 2 * NCH * 32);
+               }
+               // source rows ky .. ky+R-1 of this chunk must be split
+               for (int j = ky == 0 ? 0 : R - 1; j < R && ok; j++) ok = row_ready(j);
+               if (!ok) break;
+               // operands written by TMA or by proxy-fenced stores need no tcgen05 fence
+               uint64_t adr[R];
 #pragma unroll
-                     for (int r = 0; r < R; r++) {
-                        const int slot = slotKy + r >= g.NS ? slotKy + r - g.NS : slotKy + r;
-                        adr[r] = aD0 + (uint64_t)((slot * kSlotA + kx * 16) >> 4);
-                     }
+               for (int r = 0; r < R; r++) {
+                  const int slot = slotA + r >= g.NS ? slotA + r - g.NS : slotA + r;
+                  adr[r] = aD0 + (uint64_t)((slot * kSlotA) >> 4);
+               }
+               uint32_t acc0 = fresh0(chainStart);
+               for (int kx = 0; kx < g.KX; kx++) {
+                  if (!bSeen && !(ok = warp_wait(&bFull[d], parB))) break;
+                  const int dn = d + 1 == g.NB ? 0 : d + 1;
+                  const uint32_t parN = dn == 0 ? parB ^ 1u : parB;
 #pragma unroll
-                     for (int r = 0; r < R; r++) {
-                        const uint32_t dt = tacc + (uint32_t)(r * 2 * g.NT);
+                  for (int r = 0; r < R; r++) {
+                     const uint32_t dt = tacc + (uint32_t)(r * 2 * g.NT);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {  // K step of 8 TF32 = two chunk columns
-                           const uint64_t ah = adr[r] + k * kStepA, bhl = bd + 2 * k;
-                           mma_tf32(dt, ah, bhl, idesc, k == 0 ? acc0 : 1u);  // A_hi x [W_hi; W_lo]
-                           mma_tf32(dt, ah + kLoA, bhl, idescHi, 1);           // A_lo x W_hi
-                        }
+                     for (int k = 0; k < 4; k++) {  // K step of 8 TF32 = two chunk columns
+                        const uint64_t ah = adr[r] + k * kStepA, bhl = bd + 2 * k;
+                        mma_tf32_elect(dt, ah, bhl, idesc, k == 0 ? acc0 : 1u);  // A_hi x [W_hi; W_lo]
+                        mma_tf32_elect(dt, ah + kLoA, bhl, idescHi, 1);           // A_lo x W_hi
+                        if (r * 4 + k == 2 * R - 1) bSeen = __all_sync(0xffffffffu, mbar_try_wait(&bFull[dn], parN));
                      }
-                     mma_commit(&bEmpty[d]);
-                     cb++;
-                     if (++d == g.NB) {
-                        d = 0;
-                        bPar ^= 1u;
-                     }
+                     adr[r] += 1;  // one position (16 B) down
                   }
-                  if (!ok) break;
-                  mma_commit(&aEmpty[slotKy]);  // row ky has no later use
-                  if ((grp + 1) % g.groupsPerChain == 0 || grp + 1 == groupsPerUnit) {
-                     mma_commit(&chainFull[cc & 1]);
-                     cc++;
-                  }
+                  mma_commit_elect(&bEmpty[d]);
+                  acc0 = 1u;
+                  d = dn;
+                  parB = parN;
+                  bd = dn == 0 ? bD0 : bd + stepB;
                }
                if (!ok) break;
-               for (int j = g.KY; j < rowsPerFC; j++) mma_commit(&aEmpty[(slotBase + j) % g.NS]);
-               cbase += rowsPerFC;
-               slotBase = (slotBase + rowsPerFC) % g.NS;
+               mma_commit_elect(&aEmpty[slotA]);  // row ky has no later use
+               next_row();
+               if (--chainLeft == 0 || (ky + 1 == g.KY && fc + 1 == g.nFC)) {
+                  chainLeft = 0;
+                  mma_commit_elect(&chainFull[cc & 1]);
+                  cc++;
+               }
+            }
+            if (!ok) break;
+            for (int j = g.KY; j < rowsPerFC; j++) {
+               mma_commit_elect(&aEmpty[slotA]);
+               next_row();
             }
          }
-         // every MMA issued has completed before TMEM is released
-         mma_commit(&mmaDone);
-         mbar_wait(&mmaDone, 0);
       }
+      // every MMA issued has completed before TMEM is released
+      mma_commit_elect(&mmaDone);
+      mbar_wait(&mmaDone, 0);
    } else if (warp < 6) {
       // ================================ hi / lo split ================================
       // raw row (128-byte swizzle: chunk j of row r at r*128 + ((j ^ (r & 7)) << 4)) -> hi and lo

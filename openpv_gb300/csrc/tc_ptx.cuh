@@ -365,5 +365,24 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64
          : "memory");
 }
 
+// The same, called by a whole converged warp: one elected lane (always the same one) issues.  Nothing
+// diverges around it, so the operands can stay in uniform registers.
+__device__ __forceinline__ void mma_tf32_elect(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t accumulate) {
+   asm volatile(
+         "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n elect.sync _|e, 0xffffffff;\n"
+         " @e tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+         : "memory");
+}
+
+// mma_commit for the MMAs that the elected lane issued.
+__device__ __forceinline__ void mma_commit_elect(uint64_t *bar) {
+   asm volatile(
+         "{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+         " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar))
+         : "memory");
+}
+
 }  // namespace tc
 }  // namespace pvgpu
