@@ -400,8 +400,8 @@ pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *e
 // The tile kernel this replaces gave each warp one output row and tested every entry of its range
 // against every output: on the delivery of a V1 layer to an image (one to three features, 8x8
 // patches) seven of eight lanes had nothing to add, and one image kept 8 CTAs busy.  Measured:
-// one 16x16x64 V1 layer to 32x32x1 160 -> SB1 us; 8 x 256x256x32 spikes (2 %) to 128x128x8, 3x3 at
-// stride 2, 425 -> SEX us; 32 x 16x16x512 (5 %) to 32x32x3 754 -> SB32 us.  What bounds it is the
+// one 16x16x64 V1 layer to 32x32x1 160 -> 9 us; 8 x 256x256x32 spikes (2 %) to 128x128x8, 3x3 at
+// stride 2, 425 -> 60 us; 32 x 16x16x512 (5 %) to 32x32x3 754 -> 49 us.  What bounds it is the
 // read-add-write on shared memory (one entry's adds must land before the next one's), hence vectors of
 // up to four weights per lane, and tiles as large as the warps' copies allow -- a tile wastes what patches
 // hang over its edge -- with the entries of one tile divided over a cluster.
