@@ -599,9 +599,9 @@ def dictlearn_bench(torch, capi, reps=5):
     cpu_s = time.perf_counter() - t0
     emulated = bool(grad.emulated_fp32())
     fp32_tf = flops / (ms / 1000.0) / 1e12
-    # the emulated FP32 GEMM issues 9 BF16 products per FP32 product (each operand in three BF16
+    # the emulated FP32 GEMM issues 6 BF16 products per FP32 product (each operand in three BF16
     # parts); averaged over the whole gradient (the fold / im2col / update kernels included)
-    issued = fp32_tf * (9 if emulated else 1)
+    issued = fp32_tf * (6 if emulated else 1)
     pk = peaks()
     roofline = ({"bound": "tensor", "achieved": issued, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                  "frac": issued / pk["bf16_tflops"], "peak_source": pk.get("source", "fallback"),
