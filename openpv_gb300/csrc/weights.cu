@@ -73,21 +73,25 @@ struct HGeom {
 // feature's list with its lanes on 32 * EPT weights of the patch.  Zeros cost a lane's share of a load
 // instead of a step of every chain.  The next segment's loads are issued before the lists are walked.
 //
-// 32 images of 16x16x512 at 5 % against 32x32x3 errors, 8x8 patches: 118 us (46 M instructions, a
+// 32 images of 16x16x512 at 5 % against 32x32x3 errors, 8x8 patches: 92 us (46 M instructions, a
 // third of them the scan; the rest the walk, whose patches mostly hang over the image's edge and are
 // tested weight by weight); one thread per weight walking every position itself took 4.3 ms.
-constexpr int kSL = 16;           // loads per warp and segment
-constexpr int kMaxHWarps = 16;
+// W = the most warps a CTA has.  Patches whose weights take more than 16 warps at one weight a lane get up
+// to 32 warps of one or two weights a lane, with half the loads per warp and segment (the lists of a
+// segment stay at 128 KB): twice the chains in flight.  The call above: 118 us with 16 warps of two
+// weights, 92 with 24 of one; half the loads per segment without the warps 134; two features a CTA
+// instead of four 146 (each sector read by four CTAs).
 
 // WIDE: post activities of 2^31 values and more (64-bit offsets, computed in the walk).
-template <int EPT, int FC, bool WIDE>
-__global__ void __launch_bounds__(kMaxHWarps * 32) hebbian_kernel(HGeom g, int slabsPerCta,
+template <int EPT, int FC, int W, bool WIDE>
+__global__ void __launch_bounds__(W * 32) hebbian_kernel(HGeom g, int slabsPerCta,
                                                                   const float *__restrict__ preExt,
                                                                   const float *__restrict__ postExt,
                                                                   float *__restrict__ dw) {
-   constexpr int PL = 32 / FC;  // positions per load
+   constexpr int PL = 32 / FC;    // positions per load
+   constexpr int kSL = 256 / W;   // loads per warp and segment
    extern __shared__ __align__(16) int4 recs[];  // [FC][cap]
-   __shared__ int counts[2][kMaxHWarps][8];
+   __shared__ int counts[2][W][8];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
    const int cap = NW * kSL * PL;
    const int groups = (g.preNf + FC - 1) / FC;
@@ -271,31 +275,38 @@ __global__ void __launch_bounds__(kMaxHWarps * 32) hebbian_kernel(HGeom g, int s
    }
 }
 
-template <int EPT, int FC, bool WIDE = false>
+template <int EPT, int FC, int W, bool WIDE = false>
 pvgpu_status launch_hebbian(const HGeom &g, const float *preExt, const float *postExt, float *dw, cudaStream_t s) {
    const int slabs = (g.patchSize + 32 * EPT - 1) / (32 * EPT);
-   const int perCta = slabs < kMaxHWarps / FC ? slabs : kMaxHWarps / FC;
+   const int perCta = slabs < W / FC ? slabs : W / FC;
    const int warps = perCta * FC < 8 ? 8 : perCta * FC;  // warps beyond the lists only scan
    const int64_t gx = (int64_t)g.nkx * g.nky * ((g.preNf + FC - 1) / FC);
    const int gy = (slabs + perCta - 1) / perCta;
    if (gx > 0x7fffffff || gy > 65535) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   const size_t smem = sizeof(int4) * (size_t)warps * kSL * 32;
-   PVGPU_CUDA(cudaFuncSetAttribute(hebbian_kernel<EPT, FC, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+   const size_t smem = sizeof(int4) * (size_t)warps * (256 / W) * 32;
+   PVGPU_CUDA(cudaFuncSetAttribute(hebbian_kernel<EPT, FC, W, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
               "hebbian_dw attribute");
-   hebbian_kernel<EPT, FC, WIDE><<<dim3((unsigned)gx, gy), warps * 32, smem, s>>>(g, perCta, preExt, postExt, dw);
+   hebbian_kernel<EPT, FC, W, WIDE><<<dim3((unsigned)gx, gy), warps * 32, smem, s>>>(g, perCta, preExt, postExt, dw);
    PVGPU_CHECK_LAUNCH("hebbian_dw");
    return PVGPU_OK;
 }
 
 template <int FC>
 pvgpu_status launch_hebbian_ept(const HGeom &g, const float *preExt, const float *postExt, float *dw, cudaStream_t s) {
-   // the fewest weights per lane that a CTA's warps cover in one pass over the activity: short chains
-   // of loads behind each list entry, and more warps to hide them
-   const int per = kMaxHWarps / FC * 32;
-   if (g.patchSize <= per) return launch_hebbian<1, FC>(g, preExt, postExt, dw, s);
-   if (g.patchSize <= 2 * per) return launch_hebbian<2, FC>(g, preExt, postExt, dw, s);
-   if (g.patchSize <= 4 * per) return launch_hebbian<4, FC>(g, preExt, postExt, dw, s);
-   return launch_hebbian<8, FC>(g, preExt, postExt, dw, s);
+   // The fewest weights per lane, for short chains of loads behind each list entry and more warps to
+   // hide them, whose warps one pass over the activity serves: in one CTA, or in several where the SMs
+   // that would take them have nothing else (57 x 15x70x1 -> 32 features, 9x9 patches, 20 %: one CTA of
+   // eight weights a lane 5.8 ms, three of one 1.3).
+   const int slabs = (g.patchSize + 31) / 32;
+   const int64_t gx = (int64_t)g.nkx * g.nky * ((g.preNf + FC - 1) / FC);
+   auto fits = [&](int ept) {
+      const int per = 32 / FC * ept;
+      return slabs <= per || gx * ((slabs + per - 1) / per) <= pvgpu::num_sms();
+   };
+   if (slabs <= 16 / FC) return launch_hebbian<1, FC, 16>(g, preExt, postExt, dw, s);
+   if (fits(1)) return launch_hebbian<1, FC, 32>(g, preExt, postExt, dw, s);
+   if (fits(2)) return launch_hebbian<2, FC, 32>(g, preExt, postExt, dw, s);
+   return launch_hebbian<8, FC, 16>(g, preExt, postExt, dw, s);
 }
 
 }  // namespace
@@ -357,7 +368,7 @@ extern "C" pvgpu_status pvgpu_hebbian_dw(const pvgpu_conn_desc *conn, float dWMa
    g.nky = pre.ny > post.ny ? pre.ny / post.ny : 1;
    g.dWMax = dWMax;
    cudaStream_t s = pvgpu::as_stream(stream);
-   if (g.nPostExt * g.nb > 0x7fffffffLL) return launch_hebbian<4, 1, true>(g, preExt, postExt, dw, s);
+   if (g.nPostExt * g.nb > 0x7fffffffLL) return launch_hebbian<4, 1, 16, true>(g, preExt, postExt, dw, s);
    // features per CTA: as many as share a 32-byte sector, fewer while that leaves SMs without a CTA
    int fc = 8;
    while (fc > 1 && ((int64_t)g.nkx * g.nky * ((pre.nf + fc - 1) / fc) < 128 || fc >= 2 * pre.nf)) fc >>= 1;

@@ -17,6 +17,14 @@ CASES = [
     ((2, 32, 16, 5, 6), (8, 4, 3, 2), 4, 4, 0.3),       # many-to-one x4: sixteen kernel phases
     ((1, 8, 6, 20, 5), (32, 24, 2, 1), 16, 16, 0.2),    # one-to-many x4, halo wider than the patch needs
     ((2, 20, 12, 7, 0), (20, 12, 3, 0), 7, 7, 0.0),     # nothing active
+    ((2, 9, 7, 1, 3), (9, 7, 130, 3), 9, 9, 0.5),       # 10530 weights, one feature: eleven CTAs of 32 warps
+    ((1, 6, 5, 100, 2), (6, 5, 44, 2), 5, 5, 0.3),      # 1100 weights, a hundred features: two weights a lane
+    ((1, 6, 5, 100, 2), (6, 5, 90, 1), 5, 5, 0.3),      # 2250: eight a lane
+    ((1, 7, 6, 300, 2), (7, 6, 20, 0), 5, 5, 0.2),      # two features a CTA, 500 weights
+    ((1, 7, 6, 600, 2), (7, 6, 11, 0), 5, 5, 0.2),      # four features a CTA, 275 weights: two a lane
+    ((1, 7, 6, 1100, 2), (7, 6, 4, 2), 5, 5, 0.2),      # eight features a CTA, 100 weights
+    ((1, 7, 6, 1100, 2), (7, 6, 8, 2), 5, 5, 0.2),      # 200: two a lane
+    ((1, 7, 6, 1100, 2), (7, 6, 24, 2), 5, 5, 0.2),     # 600: eight a lane
 ]
 
 
