@@ -682,6 +682,10 @@ pvgpu_status launch_pdl(Kernel kernel, dim3 grid, int threads, size_t smem, cuda
 constexpr size_t gemm_smem(int bn) { return pvgpu::split::stages_of(bn) * 3 * (pvgpu::split::kPlaneA + (size_t)bn * 128) + 1024; }
 constexpr size_t kCorrSmem = 2 * 6 * (size_t)pvgpu::split::kPlaneA + 1024;
 
+// A band of windows takes at most this much shared memory.  The limit that a launch is checked against belongs to
+// the kernel, not to a handle, so it is set to the bound and never to one handle's size.
+constexpr size_t kBandSmem = 200 * 1024;
+
 size_t band_smem(const Geo &g) {
    return sizeof(float) * (size_t)(g.S * (kMaxBandRows - 1) + g.P) * (((g.inx + 2 * g.E) * g.C + 3) & ~3);
 }
@@ -882,7 +886,7 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
    // the split-plane path: T(0) = 0, rows of whole 16-byte groups, 32-bit matrix sizes, a band of windows in
    // shared memory
    s->tc = d->VThresh >= 0.0f && g.F % 8 == 0 && g.KP % 8 == 0 && g.M <= 0x7fffff00LL && (g.M + 127) / 128 <= 65535 &&
-           (int64_t)g.nb * g.vy <= 0x7fffffff && band_smem(g) <= 200 * 1024 &&
+           (int64_t)g.nb * g.vy <= 0x7fffffff && band_smem(g) <= kBandSmem &&
            (size_t)g.F * g.KP <= 0x7fffffff && pvgpu::encode_tiled_fn() != nullptr;
    if (s->tc) {
       auto planes = [&](bf16 **p, size_t n) { alloc(reinterpret_cast<void **>(p), 3 * n * sizeof(bf16)); };
@@ -924,8 +928,7 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
                   cudaFuncSetAttribute(pvgpu::split::corr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kCorrSmem) == cudaSuccess &&
                   with_geometry(g, [&](auto kernel) {
-                     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)std::max<size_t>(band_smem(g), 48 * 1024)) == cudaSuccess;
+                     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBandSmem) == cudaSuccess;
                   }))) {
          cudaGetLastError();
          free_all(s);
