@@ -275,6 +275,10 @@ __global__ void __launch_bounds__(W * 32) hebbian_kernel(HGeom g, int slabsPerCt
    }
 }
 
+// The lists of a CTA of W warps, the most that any launch takes.  The limit that a launch is checked against
+// belongs to the kernel, and another thread may be launching it with a smaller layer, so it is always set to this.
+constexpr size_t kListBytes = sizeof(int4) * 256 * 32;
+
 template <int EPT, int FC, int W, bool WIDE = false>
 pvgpu_status launch_hebbian(const HGeom &g, const float *preExt, const float *postExt, float *dw, cudaStream_t s) {
    const int slabs = (g.patchSize + 32 * EPT - 1) / (32 * EPT);
@@ -283,8 +287,8 @@ pvgpu_status launch_hebbian(const HGeom &g, const float *preExt, const float *po
    const int64_t gx = (int64_t)g.nkx * g.nky * ((g.preNf + FC - 1) / FC);
    const int gy = (slabs + perCta - 1) / perCta;
    if (gx > 0x7fffffff || gy > 65535) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   const size_t smem = sizeof(int4) * (size_t)warps * (256 / W) * 32;
-   PVGPU_CUDA(cudaFuncSetAttribute(hebbian_kernel<EPT, FC, W, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+   const size_t smem = kListBytes / W * warps;
+   PVGPU_CUDA(cudaFuncSetAttribute(hebbian_kernel<EPT, FC, W, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kListBytes),
               "hebbian_dw attribute");
    hebbian_kernel<EPT, FC, W, WIDE><<<dim3((unsigned)gx, gy), warps * 32, smem, s>>>(g, perCta, preExt, postExt, dw);
    PVGPU_CHECK_LAUNCH("hebbian_dw");

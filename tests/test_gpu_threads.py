@@ -1,0 +1,68 @@
+"""Host threads that call one entry point at the same time, on streams of their own, with sizes that run the
+same kernel with different amounts of shared memory: every call goes through, with the bits that one thread
+alone gets."""
+import threading
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from openpv_gb300 import build
+    build.build()
+    return torch
+
+
+def hebbian(torch, capi, seed, post_nf):
+    """3x3 patches of 4 features: 8 warps (64 KB of lists) for 18 weights, 16 (128 KB) for 504."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pre, post = capi.Loc.make(1, 12, 10, 4, 1), capi.Loc.make(1, 12, 10, post_nf, 0)
+    a = torch.randn(pre.ext_shape(), device="cuda", generator=g)
+    r = torch.randn(post.ext_shape(), device="cuda", generator=g)
+    conn = capi.conn_desc(pre, post, 3, 3)
+
+    def make():
+        dw = torch.empty(4 * 9 * post_nf, device="cuda")
+        return lambda stream: capi.hebbian_dw(conn, 0.5, a, r, dw, stream=stream), dw
+    return make
+
+
+@pytest.mark.parametrize("kernel", ["hebbian"])
+def test_same_kernel_from_several_threads(torch, kernel):
+    from openpv_gb300 import capi
+    calls = {"hebbian": lambda: [hebbian(torch, capi, 1, 56), hebbian(torch, capi, 2, 2)]}[kernel]()
+    alone = []
+    for c in calls:
+        call, out = c()
+        call(torch.cuda.current_stream())
+        alone.append(out.cpu().numpy())
+    errors, wrong, stop = [], [], time.monotonic() + 3.0
+
+    def work(i):
+        s = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(s):
+                call, out = calls[i]()
+                while time.monotonic() < stop and not errors:
+                    for _ in range(200):
+                        call(s)
+                    s.synchronize()
+                    if not np.array_equal(out.cpu().numpy().view(np.uint32), alone[i].view(np.uint32)):
+                        wrong.append(i)
+        except Exception as e:  # noqa: BLE001
+            errors.append(f"thread of size {i}: {e}")
+
+    threads = [threading.Thread(target=work, args=(i % 2,)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors and not wrong, (errors, wrong)
