@@ -406,6 +406,10 @@ pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *e
 // up to four weights per lane, and tiles as large as the warps' copies allow -- a tile wastes what patches
 // hang over its edge -- with the entries of one tile divided over a cluster.
 // -------------------------------------------------------------------------------------------
+// A plan takes at most this much shared memory.  The limit that a launch is checked against belongs to the
+// kernel, and another thread may be launching it with a smaller plan, so it is always set to the bound.
+constexpr size_t kScatSmem = 200 * 1024;
+
 struct ScatPlan {
    int TX, TY, FT, NW, cz, vec;
    int nTX, nTY, nFT;
@@ -661,7 +665,7 @@ bool scatter_plan(const PreGeom &pg, const FastGeom &g, const float *W, bool spa
          p.rowsMax = covY + sy;
          for (p.NW = 8; p.NW >= 4; p.NW >>= 1) {
             p.smem = 4 * ((size_t)p.NW * 128 + ((2 * p.rowsMax + 4) & ~3) + (size_t)p.NW * p.tileFloats);
-            if (p.smem <= 200 * 1024) break;
+            if (p.smem <= kScatSmem) break;
          }
          if (p.NW < 4) continue;
          const int64_t tiles = (int64_t)p.nTX * p.nTY * p.nFT;
@@ -690,7 +694,7 @@ pvgpu_status launch_scatter(const FastGeom &g, const ScatPlan &pl, int nb, cudaS
                             const int64_t *numActive, const float *aExt, const float *W, float *gsyn) {
    auto go = [&](auto kernel) -> pvgpu_status {
       if (pl.smem > 48 * 1024)
-         PVGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem),
+         PVGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScatSmem),
                     "deliver_pre scatter attribute");
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -34,10 +34,33 @@ def hebbian(torch, capi, seed, post_nf):
     return make
 
 
-@pytest.mark.parametrize("kernel", ["hebbian"])
+def scatter(torch, capi, seed, nb, n, nf):
+    """5x5 patches of 12 features: tiles of 62 KB for the small layer, of 112 KB for the large one."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pre, post = capi.Loc.make(nb, n, n, nf, 2), capi.Loc.make(nb, n, n, 12, 0)
+    a = torch.randn(pre.ext_shape(), device="cuda", generator=g)
+    a *= torch.rand(pre.ext_shape(), device="cuda", generator=g) < 0.01
+    e = torch.empty(nb, pre.num_ext, dtype=torch.int64, device="cuda")
+    num = torch.zeros(nb, dtype=torch.int64, device="cuda")
+    capi.compact_active(a, nb, pre.num_ext, e, num)
+    w = torch.randn(nf * 25 * 12, device="cuda", generator=g)
+    conn = capi.conn_desc(pre, post, 5, 5)
+
+    def make():
+        gs = torch.empty(post.res_shape(), device="cuda")
+
+        def call(stream):
+            gs.zero_()
+            capi.deliver_pre(conn, w, gs, entries=e, num_active=num, stream=stream)
+        return call, gs
+    return make
+
+
+@pytest.mark.parametrize("kernel", ["hebbian", "scatter"])
 def test_same_kernel_from_several_threads(torch, kernel):
     from openpv_gb300 import capi
-    calls = {"hebbian": lambda: [hebbian(torch, capi, 1, 56), hebbian(torch, capi, 2, 2)]}[kernel]()
+    calls = {"hebbian": lambda: [hebbian(torch, capi, 1, 56), hebbian(torch, capi, 2, 2)],
+             "scatter": lambda: [scatter(torch, capi, 1, 4, 64, 64), scatter(torch, capi, 2, 2, 32, 16)]}[kernel]()
     alone = []
     for c in calls:
         call, out = c()
