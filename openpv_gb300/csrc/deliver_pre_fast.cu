@@ -362,12 +362,13 @@ pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *e
    const int64_t gx = (int64_t)((g.postNx + kCols - 1) / kCols) * slabs;
    // rows per CTA: a CTA also visits the nyp - 1 presynaptic rows around its own, so the cost is the
    // CTAs per SM times RS + nyp - 1, and more where an SM has too few CTAs (8 warps each) to hide
-   // their loads.  16 x 128x128x256 -> 64, 7x7, 1 % active: 545 / 504 / 469 / 606 us at 16 / 32 / 64
-   // / 128 rows.
+   // their loads; no more than the row table holds, which 64 rows of a layer four times as fine exceed.
+   // 16 x 128x128x256 -> 64, 7x7, 1 % active: 545 / 504 / 469 / 606 us at 16 / 32 / 64 / 128 rows.
    const int occ = fpl * g.nyp > 16 ? 2 : 4;
-   int RS = 4;
+   const int rowsPer = pg.pre.ny > pg.post.ny ? pg.pre.ny / pg.post.ny : 1;
+   int RS = 0;
    double best = 1e300;
-   for (int r = 4; r <= 64; r *= 2) {
+   for (int r = 4; r <= 64 && (r + g.nyp) * rowsPer <= kRowsMax; r *= 2) {
       const double perSm = std::max(1.0, (double)gx * ((g.postNy + r - 1) / r) * pg.pre.nb / num_sms());
       const double cost = perSm * (r + g.nyp - 1) * (1.0 + 1.5 / std::min(perSm, (double)occ));
       if (cost < best) {
@@ -375,8 +376,7 @@ pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *e
          RS = r;
       }
    }
-   const int rowsPer = pg.pre.ny > pg.post.ny ? pg.pre.ny / pg.post.ny : 1;
-   if ((RS + g.nyp) * rowsPer > kRowsMax) return PVGPU_ERR_UNSUPPORTED_SHAPE;
+   if (RS == 0) return PVGPU_ERR_UNSUPPORTED_SHAPE;
    const int gy = (g.postNy + RS - 1) / RS;
    if (gx > 0x7fffffff || gy > 65535) return PVGPU_ERR_UNSUPPORTED_SHAPE;
    const dim3 grid((unsigned)gx, gy, pg.pre.nb);
