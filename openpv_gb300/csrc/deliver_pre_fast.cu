@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace {
@@ -349,40 +350,100 @@ pvgpu_status launch_cols_nyp(const FastGeom &g, dim3 grid, int RS, cudaStream_t 
    return PVGPU_ERR_UNSUPPORTED_SHAPE;
 }
 
-pvgpu_status try_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *entries, const int64_t *numActive,
-                      const float *aExt, const float *W, float *gsyn, cudaStream_t s) {
-   if (g.nyp > 16) return PVGPU_ERR_UNSUPPORTED_SHAPE;
+// One launch of the column kernel: features per lane, slabs of 32 * fpl features, rows and CTAs per SM of a
+// CTA, and its estimated cycles.
+struct ColPlan {
+   int fpl, slabs, RS, occ;
+   double cost;
+};
+
+// Activity that the estimates of both kernels assume (the result does not depend on it).
+double assumed_density(bool sparse) { return sparse ? 0.05 : 0.3; }
+
+// g.nyp: the patch rows of the pass.  false for a shape that the kernel does not take.
+bool cols_plan(const PreGeom &pg, const FastGeom &g, const float *W, const float *gsyn, bool sparse, ColPlan *p) {
    // features per lane: the fewest slabs of 32 * FPL features whose vector loads are aligned (a
    // weight row starts at a multiple of nfp floats)
    const uintptr_t al = reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(gsyn);
    const int maxFpl = g.nyp > 9 ? 2 : 4;
    int fpl = 1;
    while (fpl < maxFpl && 32 * fpl < g.nfp && g.nfp % (2 * fpl) == 0 && al % (8 * fpl) == 0) fpl *= 2;
-   const int slabs = (g.nfp + 32 * fpl - 1) / (32 * fpl);
-   const int64_t gx = (int64_t)((g.postNx + kCols - 1) / kCols) * slabs;
+   p->fpl = fpl;
+   p->slabs = (g.nfp + 32 * fpl - 1) / (32 * fpl);
+   const int64_t gx = (int64_t)((g.postNx + kCols - 1) / kCols) * p->slabs;
    // rows per CTA: a CTA also visits the nyp - 1 presynaptic rows around its own, so the cost is the
    // CTAs per SM times RS + nyp - 1, and more where an SM has too few CTAs (8 warps each) to hide
    // their loads; no more than the row table holds, which 64 rows of a layer four times as fine exceed.
    // 16 x 128x128x256 -> 64, 7x7, 1 % active: 545 / 504 / 469 / 606 us at 16 / 32 / 64 / 128 rows.
-   const int occ = fpl * g.nyp > 16 ? 2 : 4;
+   p->occ = fpl * g.nyp > 16 ? 2 : 4;
    const int rowsPer = pg.pre.ny > pg.post.ny ? pg.pre.ny / pg.post.ny : 1;
-   int RS = 0;
    double best = 1e300;
+   p->RS = 0;
    for (int r = 4; r <= 64 && (r + g.nyp) * rowsPer <= kRowsMax; r *= 2) {
       const double perSm = std::max(1.0, (double)gx * ((g.postNy + r - 1) / r) * pg.pre.nb / num_sms());
-      const double cost = perSm * (r + g.nyp - 1) * (1.0 + 1.5 / std::min(perSm, (double)occ));
+      const double cost = perSm * (r + g.nyp - 1) * (1.0 + 1.5 / std::min(perSm, (double)p->occ));
       if (cost < best) {
          best = cost;
-         RS = r;
+         p->RS = r;
       }
    }
-   if (RS == 0) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   const int gy = (g.postNy + RS - 1) / RS;
-   if (gx > 0x7fffffff || gy > 65535) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   const dim3 grid((unsigned)gx, gy, pg.pre.nb);
-   return fpl == 1   ? launch_cols_nyp<1>(g, grid, RS, s, entries, numActive, aExt, W, gsyn)
-          : fpl == 2 ? launch_cols_nyp<2>(g, grid, RS, s, entries, numActive, aExt, W, gsyn)
-                     : launch_cols_nyp<4>(g, grid, RS, s, entries, numActive, aExt, W, gsyn);
+   if (p->RS == 0) return false;
+   const int gy = (g.postNy + p->RS - 1) / p->RS;
+   if (gx > 0x7fffffff || gy > 65535) return false;
+   // entries of a presynaptic row that one column takes, and 32-entry chunks that its warp reads for them
+   const double perCol = (double)pg.pre.nx / pg.post.nx * g.nf * assumed_density(sparse);
+   const double took = g.nxp * perCol, read = (kCols + g.nxp - 1) * perCol, chunks = read / 32 + 1 - std::exp(-read);
+   const double perEntry = 1 + g.nyp * (1 + std::max(1.0, fpl / 2.0));
+   const double rows = (double)(std::min(p->RS, g.postNy) + g.nyp - 1) * pg.pre.ny / pg.post.ny;
+   const double ctas = (double)gx * gy * pg.pre.nb;
+   const double instr = rows * (33 + 22 * chunks + took * perEntry) + 64;
+   const double serial = rows * (900 + 870 * chunks + took / 2 * (280 + 2 * perEntry));
+   p->cost = std::max(ctas * std::min(g.postNx, kCols) * instr / (num_sms() * 0.62),
+                      serial * std::max(1.0, ctas / ((double)num_sms() * p->occ)));
+   return true;
+}
+
+// Patches taller than the window of 16 rows go in passes of equal heights, each a delivery of its own.
+constexpr int kWindow = 16;
+
+FastGeom cols_part(const FastGeom &g, int pass, int *ky0) {
+   const int passes = (g.nyp + kWindow - 1) / kWindow;
+   FastGeom q = g;
+   *ky0 = (int)((int64_t)g.nyp * pass / passes);
+   q.nyp = (int)((int64_t)g.nyp * (pass + 1) / passes) - *ky0;
+   q.ay.o += *ky0;
+   return q;
+}
+
+// The estimate of all passes; false where the kernel does not take one of them.
+bool cols_cost(const PreGeom &pg, const FastGeom &g, const float *W, const float *gsyn, bool sparse, double *cost) {
+   *cost = 0;
+   for (int i = 0; i < (g.nyp + kWindow - 1) / kWindow; i++) {
+      int ky0;
+      ColPlan p;
+      const FastGeom q = cols_part(g, i, &ky0);
+      if (!cols_plan(pg, q, W, gsyn, sparse, &p)) return false;
+      *cost += p.cost;
+   }
+   return true;
+}
+
+// One pass, or several that cols_cost has accepted: nothing is launched for a shape that the kernel does not take.
+pvgpu_status run_cols(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *entries, const int64_t *numActive,
+                      const float *aExt, const float *W, float *gsyn, cudaStream_t s) {
+   for (int i = 0; i < (g.nyp + kWindow - 1) / kWindow; i++) {
+      int ky0;
+      ColPlan p;
+      const FastGeom q = cols_part(g, i, &ky0);
+      if (!cols_plan(pg, q, W, gsyn, entries != nullptr, &p)) return PVGPU_ERR_UNSUPPORTED_SHAPE;
+      const dim3 grid((unsigned)((g.postNx + kCols - 1) / kCols * p.slabs), (g.postNy + p.RS - 1) / p.RS, pg.pre.nb);
+      const float *Wp = W + (size_t)ky0 * g.nxp * g.nfp;
+      const pvgpu_status r = p.fpl == 1   ? launch_cols_nyp<1>(q, grid, p.RS, s, entries, numActive, aExt, Wp, gsyn)
+                             : p.fpl == 2 ? launch_cols_nyp<2>(q, grid, p.RS, s, entries, numActive, aExt, Wp, gsyn)
+                                          : launch_cols_nyp<4>(q, grid, p.RS, s, entries, numActive, aExt, Wp, gsyn);
+      if (r != PVGPU_OK) return r;
+   }
+   return PVGPU_OK;
 }
 
 // -------------------------------------------------------------------------------------------
@@ -673,7 +734,7 @@ bool scatter_plan(const PreGeom &pg, const FastGeom &g, const float *W, bool spa
          const int vectors = (g.nyp * g.nxp * p.FT / p.vec + 31) / 32;
          // a vector of one entry: load, read, multiply-adds, write; serially a read-add-write's latency
          const double perEntry = 18 + vectors * (4.0 + p.vec), latency = 45 + vectors * (4.0 + 2.0 * p.vec);
-         const double E = (double)covX * covY * g.nf * (sparse ? 0.05 : 0.3) + 1.0;
+         const double E = (double)covX * covY * g.nf * assumed_density(sparse) + 1.0;
          const double outs = (double)p.TX * p.TY * p.FT / 32;
          for (p.cz = 1; p.cz <= 8; p.cz *= 2) {
             if (tiles * p.cz > 0x7fffffff || (p.cz > 1 && E / p.cz < 64)) break;
@@ -726,10 +787,28 @@ pvgpu_status scatter_vec(const FastGeom &g, const ScatPlan &pl, int nb, cudaStre
    return launch_scatter<4, VEC == 4 ? 2 : 4, VEC>(g, pl, nb, s, entries, numActive, aExt, W, gsyn);
 }
 
-pvgpu_status try_scatter(const PreGeom &pg, const FastGeom &g, const pvgpu_entry *entries, const int64_t *numActive,
-                         const float *aExt, const float *W, float *gsyn, cudaStream_t s) {
-   ScatPlan pl;
-   if (!scatter_plan(pg, g, W, entries != nullptr, &pl)) return PVGPU_ERR_UNSUPPORTED_SHAPE;
+// The chosen plan's cycles on the scale of ColPlan::cost: as in scatter_plan, but with the decoding of a large
+// patch's blocks and the latencies as 1,000 measured geometries have them.
+double scatter_cost(const PreGeom &pg, const FastGeom &g, bool sparse, const ScatPlan &p) {
+   const int sx = std::max(1, pg.pre.nx / pg.post.nx), sy = std::max(1, pg.pre.ny / pg.post.ny);
+   const int tx = std::max(1, pg.post.nx / pg.pre.nx), ty = std::max(1, pg.post.ny / pg.pre.ny);
+   const int vectors = (g.nyp * g.nxp * p.FT / p.vec + 31) / 32, ept = std::min(vectors, 4);
+   const double cov = ((double)(p.TX + g.nxp - 1) * sx / tx) * ((double)(p.TY + g.nyp - 1) * sy / ty);
+   const double E = cov * g.nf * assumed_density(sparse) + 1.0, warps = (double)p.cz * p.NW;
+   const double chunks = std::max(E / 32, std::min(E, warps));
+   const double perChunk = 2 + (vectors > ept ? (vectors + ept - 1) / ept * ept * 200.0 : 0.0);
+   const double outs = (double)p.TX * p.TY * p.FT / 32;
+   const double instr = E / p.cz * (28 + vectors * (13.3 + p.vec)) + chunks / p.cz * perChunk +
+                        p.NW * (p.tileFloats / 128.0 + 900) + outs * (p.NW * 2 + 8 + (p.cz > 1 ? 20 : 0));
+   const double serial = 4800 + std::max(1.0, E / warps) * (210 + vectors * (23.0 + 2 * p.vec)) +
+                         std::max(1.0, chunks / warps) * perChunk * 6.9 + p.tileFloats / 64.0 + outs * 4 + (p.cz > 1 ? 4000 : 0);
+   const double n = (double)p.nTX * p.nTY * p.nFT * p.cz * pg.pre.nb, sms = num_sms();
+   const int occ = (int)std::min<size_t>(2048 / (p.NW * 32), (227 * 1024) / (p.smem + 1024));
+   return std::max(n * instr / (sms * 1.46), serial * std::max(1.0, n / (sms * occ)));
+}
+
+pvgpu_status run_scatter(const PreGeom &pg, const FastGeom &g, const ScatPlan &pl, const pvgpu_entry *entries,
+                         const int64_t *numActive, const float *aExt, const float *W, float *gsyn, cudaStream_t s) {
    const int nb = pg.pre.nb;
    return pl.vec == 4   ? scatter_vec<4>(g, pl, nb, s, entries, numActive, aExt, W, gsyn)
           : pl.vec == 2 ? scatter_vec<2>(g, pl, nb, s, entries, numActive, aExt, W, gsyn)
@@ -738,16 +817,32 @@ pvgpu_status try_scatter(const PreGeom &pg, const FastGeom &g, const pvgpu_entry
 
 }  // namespace
 
-// Which kernel: with 24 post features or more a column's lanes are at least three quarters full and
-// its accumulators stay in registers; below that the lanes of the scatter kernel are.
+// Which kernel: with 24 post features or more and a patch that fits the window, a column's lanes are at least
+// three quarters full and its accumulators stay in registers.  Else the scatter kernel, whose lanes are the
+// weights of a patch -- unless no plan for it exists, or the patch is so large that a tile is mostly margin (25 x
+// 23 weights of 21 features on tiles of 16 x 16 x 3: every entry is added to 41 of them); then columns, where the
+// scatter kernel would take 20 us and more and their estimate is 1.5 times lower.  (Both lines keep close calls
+// with the scatter kernel: over 2,000 geometries with patches of up to 33 x 33 the pick is within 3 to 8 % of the
+// faster of the two on average.)  12 x 122x40x40 -> 138, 23x21 patches, 0.6 % active: scatter 75 ms, the tile
+// kernel 1.9, columns 0.46; 9 x 57x73x17 -> 21, 25x23: 2.4, 0.76, 0.26 ms; 2 x 11x5x206 -> 53, 9x19: 51, 623,
+// 102 us.
 pvgpu_status pvgpu::deliver_pre_fast(const PreGeom &pg, const pvgpu_entry *entries, const int64_t *numActive,
                                      const float *aExt, const float *W, float *gsyn, cudaStream_t s) {
    // 32-bit offsets inside an image's activity and inside the weights
    const int64_t weights = (int64_t)pg.nkx * pg.nky * pg.nkf * pg.patchSize;
    if (pg.pre.numExt() > 0x7fffffffLL || weights > 0x7fffffffLL) return PVGPU_ERR_UNSUPPORTED_SHAPE;
    const FastGeom g = fast_geom(pg);
-   pvgpu_status r = PVGPU_ERR_UNSUPPORTED_SHAPE;
-   if (pg.nfp >= 24) r = try_cols(pg, g, entries, numActive, aExt, W, gsyn, s);
-   if (r == PVGPU_ERR_UNSUPPORTED_SHAPE) r = try_scatter(pg, g, entries, numActive, aExt, W, gsyn, s);
-   return r;
+   const bool sparse = entries != nullptr;
+   if (g.nfp >= 24 && g.nyp <= kWindow) {
+      const pvgpu_status r = run_cols(pg, g, entries, numActive, aExt, W, gsyn, s);
+      if (r != PVGPU_ERR_UNSUPPORTED_SHAPE) return r;
+   }
+   ScatPlan pl;
+   const bool takesScatter = scatter_plan(pg, g, W, sparse, &pl);
+   const double scatter = takesScatter ? scatter_cost(pg, g, sparse, pl) : 1e300;
+   double cols;
+   if (scatter > 40000 && cols_cost(pg, g, W, gsyn, sparse, &cols) && 1.5 * cols < scatter)
+      return run_cols(pg, g, entries, numActive, aExt, W, gsyn, s);
+   if (takesScatter) return run_scatter(pg, g, pl, entries, numActive, aExt, W, gsyn, s);
+   return PVGPU_ERR_UNSUPPORTED_SHAPE;
 }
