@@ -962,7 +962,8 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
    alloc(reinterpret_cast<void **>(&s->sGD), (size_t)K * nR * 4);
    alloc(reinterpret_cast<void **>(&s->WT), (size_t)g.F * g.KP * 4);
    alloc(reinterpret_cast<void **>(&s->R), nR * 4);
-   alloc(reinterpret_cast<void **>(&s->Z), nV * 4);
+   constexpr int kProbe = 16;  // the probe below multiplies two kProbe x kProbe blocks within Z
+   alloc(reinterpret_cast<void **>(&s->Z), std::max<size_t>(nV, 2 * kProbe * kProbe) * 4);
    alloc(reinterpret_cast<void **>(&s->gR), nR * 4);
    alloc(reinterpret_cast<void **>(&s->gD), nR * 4);
    alloc(reinterpret_cast<void **>(&s->gA), nV * 4);
@@ -992,9 +993,9 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
       float *p = s->Z;
       const float one = 1.0f, zero = 0.0f;
       g_blas.setStream(s->blas, nullptr);
-      if (g_blas.gemmEx(s->blas, CUBLAS_OP_N, CUBLAS_OP_N, 16, 16, 16, &one, p, CUDA_R_32F, 16, p, CUDA_R_32F, 16, &zero,
-                        p + 256, CUDA_R_32F, 16, CUBLAS_COMPUTE_32F_EMULATED_16BFX9, CUBLAS_GEMM_DEFAULT) !=
-          CUBLAS_STATUS_SUCCESS)
+      if (g_blas.gemmEx(s->blas, CUBLAS_OP_N, CUBLAS_OP_N, kProbe, kProbe, kProbe, &one, p, CUDA_R_32F, kProbe, p, CUDA_R_32F,
+                        kProbe, &zero, p + kProbe * kProbe, CUDA_R_32F, kProbe, CUBLAS_COMPUTE_32F_EMULATED_16BFX9,
+                        CUBLAS_GEMM_DEFAULT) != CUBLAS_STATUS_SUCCESS)
          s->compute = CUBLAS_COMPUTE_32F;
       cudaDeviceSynchronize();
       cudaGetLastError();
