@@ -397,9 +397,9 @@ pvgpu_status pvgpu_cost_sum(
  * V1 -> error weights), x: device FP32 [nbatch][inNy][inNx][inNf]; dW (same layout as W) and
  * *loss (device double) are overwritten.  The deliveries and their adjoints are GEMMs over
  * im2col'd operands: FP32 emulated on the BF16 tensor cores by the library's own kernels where
- * v1Nf and nxp * nxp * inNf are multiples of 8 (dW and *loss come out NaN if a bounded device wait
- * gives up; never expected), else by cuBLAS, which emulates it or runs plain FP32
- * (pvgpu_lca_grad_info tells).  The rest is the library's own kernels; a run is one CUDA
+ * v1Nf and nxp * nxp * inNf are multiples of 8 and their buffers fit in the free memory (dW and *loss
+ * come out NaN if a bounded device wait gives up; never expected), else by cuBLAS, which emulates it or
+ * runs plain FP32 (pvgpu_lca_grad_info tells).  The rest is the library's own kernels; a run is one CUDA
  * graph, captured at the first run with a given set of pointers (make that run outside any
  * stream capture) and replayed on `stream`.  create returns PVGPU_ERR_UNSUPPORTED_SHAPE when
  * cuBLAS is needed and cannot be loaded. */

@@ -885,7 +885,8 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
    f32(&s->ck, (size_t)s->nseg * nV);
    // the split-plane path: T(0) = 0, rows of whole 16-byte groups, 32-bit matrix sizes, a band of windows in
    // shared memory
-   s->tc = d->VThresh >= 0.0f && g.F % 8 == 0 && g.KP % 8 == 0 && g.M <= 0x7fffff00LL && (g.M + 127) / 128 <= 65535 &&
+   bool noRoom = false;
+   s->tc = ok && d->VThresh >= 0.0f && g.F % 8 == 0 && g.KP % 8 == 0 && g.M <= 0x7fffff00LL && (g.M + 127) / 128 <= 65535 &&
            (int64_t)g.nb * g.vy <= 0x7fffffff && band_smem(g) <= kBandSmem &&
            (size_t)g.F * g.KP <= 0x7fffffff && pvgpu::encode_tiled_fn() != nullptr;
    if (s->tc) {
@@ -934,22 +935,32 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
          free_all(s);
          return pvgpu::record_message(PVGPU_ERR_LAUNCH, "lca_grad: tensor maps");
       }
-      if (!ok) {
-         cudaGetLastError();
-         free_all(s);
-         return PVGPU_ERR_OOM;
+      if (ok) {
+         if (cudaStreamCreateWithFlags(&s->capStream, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaGetLastError();
+            s->capStream = nullptr;
+         }
+         *out = s;
+         return PVGPU_OK;
       }
-      if (cudaStreamCreateWithFlags(&s->capStream, cudaStreamNonBlocking) != cudaSuccess) {
-         cudaGetLastError();
-         s->capStream = nullptr;
+      // The low parts of the checkpoints are half as much again (100 steps with a checkpoint before each: 644 bytes a
+      // neuron against 440): where only the library path's buffers fit, that path runs.
+      cudaGetLastError();
+      void **mine[] = {(void **)&s->V[0], (void **)&s->A[0], (void **)&s->sV,  (void **)&s->ckLo, (void **)&s->vLo,
+                       (void **)&s->sVLo, (void **)&s->pA,   (void **)&s->pR,  (void **)&s->pG,   (void **)&s->pGD,
+                       (void **)&s->pW,   (void **)&s->pWT,  (void **)&s->P,   (void **)&s->err};
+      for (void **p : mine) {
+         if (*p) cudaFree(*p);
+         *p = nullptr;
       }
-      *out = s;
-      return PVGPU_OK;
+      s->tc = false;
+      ok = noRoom = true;
    }
    std::call_once(g_blas_once, load_blas);
    if (!g_blas.ok) {
       free_all(s);
-      return pvgpu::record_message(PVGPU_ERR_UNSUPPORTED_SHAPE, "lca_grad: cuBLAS could not be loaded");
+      return noRoom ? PVGPU_ERR_OOM
+                    : pvgpu::record_message(PVGPU_ERR_UNSUPPORTED_SHAPE, "lca_grad: cuBLAS could not be loaded");
    }
    for (int i = 0; i < 2; i++) {
       alloc(reinterpret_cast<void **>(&s->V[i]), nV * 4);

@@ -48,3 +48,12 @@ def test_library_path_probe_stays_in_its_buffer(create):
              line(2, (64, 64, 1), (16, 16, 20), 16, 4, 2)]
     for got in create(*cases):
         assert got[:2] == (OK, 0) and got[3:] == (0, 0), got
+
+
+def test_library_path_where_the_split_plane_one_does_not_fit(create):
+    """100 steps with a checkpoint before each: 2.7 GB on the split-plane path, 1.9 on the other."""
+    case = lambda mb: line(8, (32, 32, 1), (16, 16, 2048), 8, 100, 1, budget_mb=mb)  # noqa: E731
+    roomy, tight, short = create(case(3000), case(2300), case(1500))
+    assert roomy[:2] == (OK, 0) and roomy[3:] == (0, 1) and roomy[2] > 2300
+    assert tight[:2] == (OK, 0) and tight[3:] == (0, 0) and tight[2] <= 2300
+    assert short[:2] == (OOM, 0) and short[3] == 0
