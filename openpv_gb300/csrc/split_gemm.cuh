@@ -122,6 +122,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    griddep_launch_dependents();
    griddep_wait();
    bool ok = true;
+   int issued = 0;  // the load lane's copies
    constexpr int HALF = BN / 2, RUN = HALF < 32 ? HALF : 32;  // an epilogue warp's columns, columns per TMEM load
    auto load_run = [](uint32_t at, float *v) {
       if constexpr (RUN == 32) tmem_ld32(at, v);
@@ -130,7 +131,6 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    float acc[HALF];
    if (warp == kEpiWarps) {
       if (lane == 0) {
-         int issued = 0;
          for (int c = 0; c < chunks && ok; c++) {
             const int s = c % kStages, u = c / kStages;
             if (u > 0 && !(ok = mbar_wait(&empty[s], (uint32_t)((u - 1) & 1)))) break;
@@ -138,9 +138,6 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
             load(c, smem + s * stageBytes, &full[s]);
             issued = c + 1;
          }
-         if (!ok)
-            for (int c = issued > kStages ? issued - kStages : 0; c < issued; c++)
-               mbar_wait(&full[c % kStages], (uint32_t)((c / kStages) & 1));
       }
    } else if (warp == kEpiWarps + 1) {
       if (lane == 0) {
@@ -195,6 +192,11 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    float *z = reinterpret_cast<float *>(smem);  // the stages are free: every MMA is done
    if (!good) {
       if (threadIdx.x == 0) atomicExch(err, 1);
+      // copies still in flight land before the CTA may exit, whichever role gave up: this one may have issued all
+      // of its own and gone on
+      if (warp == kEpiWarps && lane == 0)
+         for (int c = issued > kStages ? issued - kStages : 0; c < issued; c++)
+            mbar_wait(&full[c % kStages], (uint32_t)((c / kStages) & 1));
    } else if (warp < kEpiWarps) {
       const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * BN + (warp >> 2) * HALF;
       float *zr = z + (size_t)((warp & 3) * 32 + lane) * LZ + (warp >> 2) * HALF;
