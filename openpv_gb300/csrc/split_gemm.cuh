@@ -90,6 +90,18 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
    return p + ((1024u - (a & 1023u)) & 1023u);
 }
 
+// A wait of a kernel of a run: at most kWaitNs, and no longer than a look at the run's error word where it is set,
+// so that a run whose first wait gave up ends at once and not after a limit for each of its kernels.
+__device__ __forceinline__ bool run_wait(uint64_t *bar, uint32_t parity, const int *err) {
+   if (mbar_try_wait(bar, parity)) return true;
+   const uint64_t t0 = global_ns();
+   for (;;) {
+      for (int i = 0; i < 64; i++)
+         if (mbar_try_wait(bar, parity)) return true;
+      if (*reinterpret_cast<const volatile int *>(err) || global_ns() - t0 > kWaitNs) return false;
+   }
+}
+
 // The loads, MMAs and epilogue that the two kernels below share: `chunks` stages of operand planes, loaded
 // by load(chunk, stage base, full barrier), each multiplied in two halves of K: mma(stage base, half, product,
 // accumulator, accumulate).  TMEM columns: the two p0 q0 accumulators, then the small products'.
@@ -109,6 +121,9 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
                                          uint64_t *bars, Load load, Mma mma, Early early, Late late, Rows rows) {
    uint64_t *full = bars, *empty = full + kStages, *accFull = empty + kStages, *accEmpty = accFull + 2, *done = accEmpty + 2;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   // a run that has failed loads nothing more (read here, so that the barriers' set-up hides the latency: a failure
+   // of the kernel just before may go unseen)
+   bool ok = !(warp == kEpiWarps && lane == 0 && *reinterpret_cast<const volatile int *>(err) != 0);
    if (threadIdx.x == 0) {
       for (int i = 0; i < bars_of<kStages>(); i++)
          mbar_init(&bars[i], &bars[i] == accEmpty || &bars[i] == accEmpty + 1 ? kEpiWarps : 1);
@@ -121,7 +136,6 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    const uint32_t tmem = *tmemBase;
    griddep_launch_dependents();
    griddep_wait();
-   bool ok = true;
    int issued = 0;  // the load lane's copies
    constexpr int HALF = BN / 2, RUN = HALF < 32 ? HALF : 32;  // an epilogue warp's columns, columns per TMEM load
    auto load_run = [](uint32_t at, float *v) {
@@ -133,7 +147,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
       if (lane == 0) {
          for (int c = 0; c < chunks && ok; c++) {
             const int s = c % kStages, u = c / kStages;
-            if (u > 0 && !(ok = mbar_wait(&empty[s], (uint32_t)((u - 1) & 1)))) break;
+            if (u > 0 && !(ok = run_wait(&empty[s], (uint32_t)((u - 1) & 1), err))) break;
             mbar_arrive_expect_tx(&full[s], stageBytes);
             load(c, smem + s * stageBytes, &full[s]);
             issued = c + 1;
@@ -143,13 +157,13 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
       if (lane == 0) {
          for (int c = 0; c < chunks && ok; c++) {
             const int s = c % kStages;
-            if (!(ok = mbar_wait(&full[s], (uint32_t)((c / kStages) & 1)))) break;
+            if (!(ok = run_wait(&full[s], (uint32_t)((c / kStages) & 1), err))) break;
             tc_fence_after();
             const uint32_t st = smem_u32(smem + s * stageBytes);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                // chain 2 c + h, accumulator h, once the epilogue has read the chain before in it
-               if (c > 0 && !(ok = mbar_wait(&accEmpty[h], (uint32_t)((c - 1) & 1)))) break;
+               if (c > 0 && !(ok = run_wait(&accEmpty[h], (uint32_t)((c - 1) & 1), err))) break;
                tc_fence_after();
                mma(st, 2 * h, 0, tmem + h * BN, 0u);
                mma(st, 2 * h + 1, 0, tmem + h * BN, 1u);
@@ -171,7 +185,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
       const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * HALF;
 #pragma unroll 1
       for (int d = 0; d < 2 * chunks && ok; d++) {
-         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&accFull[d & 1], (uint32_t)((d >> 1) & 1))))) break;
+         if (!(ok = __all_sync(0xffffffffu, run_wait(&accFull[d & 1], (uint32_t)((d >> 1) & 1), err)))) break;
          tc_fence_after();
 #pragma unroll
          for (int c = 0; c < HALF; c += RUN) {

@@ -5,7 +5,8 @@ with a random scheduler between the roles, copies that land in any order and com
 Without a late copy a run must end with every role done, every barrier on a phase boundary and no wait that saw
 a barrier more than one phase away.  With copies that are late, every wait is bounded: when nothing can move on,
 the limit passes and the waits open at that moment give up.  Whatever is late then, the CTA must not exit with a
-copy in flight, unless the wait for that very copy ran out as well."""
+copy in flight, unless the wait for that very copy ran out as well.  And a run of many such kernels, of which one
+has given up, must end without a limit for each of the others."""
 import random
 
 import pytest
@@ -14,11 +15,13 @@ EPI = 8
 
 
 class Cta:
-    """One CTA.  late: copies (chunk numbers) that land only after `after` limits have passed."""
+    """One CTA.  late: copies (chunk numbers) that land only after `after` limits have passed.  failed: the run's
+    error word on entry, which the load lane reads first and the other waits when they are not over at once."""
 
-    def __init__(self, chunks, stages, seed, late=(), after=1, drain_all=True):
+    def __init__(self, chunks, stages, seed, late=(), after=1, drain_all=True, failed=False):
         self.chunks, self.stages, self.rnd = chunks, stages, random.Random(seed)
         self.late, self.after, self.drain_all = set(late), after, drain_all
+        self.failed = failed
         self.limits = 0  # limits that passed
         self.gen = 0
         self.count, self.pending, self.done = {}, {}, {}
@@ -51,7 +54,7 @@ class Cta:
                 self.aliased.append((name, k, d))
             if (d & 1) != (k & 1):
                 return True
-            if self.gen != gen:
+            if self.gen != gen or (self.failed and name != "done"):
                 return False
             yield "blocked"
 
@@ -61,8 +64,8 @@ class Cta:
                 self.landing_given_up += 1
 
     def load(self):
-        ok, issued = True, 0
-        for c in range(self.chunks):
+        ok, issued = not self.failed, 0
+        for c in range(self.chunks if ok else 0):
             s, u = c % self.stages, c // self.stages
             if u and not (yield from self.wait(f"empty{s}", u - 1)):
                 ok = False
@@ -171,6 +174,22 @@ def test_no_copy_in_flight_at_exit(chunks, stages):
                 assert not c.commits and c.in_flight() <= c.landing_given_up
                 if after == 1:
                     assert c.in_flight() == 0, (late, seed)
+
+
+@pytest.mark.parametrize("chunks, stages", SHAPES)
+def test_a_failed_run_ends_promptly(chunks, stages):
+    """Copies that never land, from the first of forty kernels on: one limit for its waits and one for each copy it
+    has in flight, none for the kernels after it -- and one and more for each where the error word is not read."""
+    def run(reads):
+        limits, failed = 0, False
+        for k in range(40):
+            c = Cta(chunks, stages, k, range(chunks), 1 << 30, failed=failed and reads)
+            failed = not c.run() or failed
+            limits += c.limits
+            assert not c.commits and c.in_flight() <= c.landing_given_up
+        return limits
+    assert run(True) <= 1 + stages
+    assert run(False) >= 40
 
 
 def test_a_drain_by_the_load_lane_alone_is_caught():
