@@ -90,6 +90,13 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
    return p + ((1024u - (a & 1023u)) & 1023u);
 }
 
+// The last copies of `chunks` stages land.  Out of line: a healthy run never calls it, and inlined it costs the
+// gradient 4 % through what the compiler then makes of the rest (32 x 64x64x1 -> 16x16x256, 100 steps: 11.23 ms, now
+// 10.81).
+static __device__ __noinline__ void land(uint64_t *full, int stages, int chunks) {
+   for (int c = chunks > stages ? chunks - stages : 0; c < chunks; c++) mbar_wait(&full[c % stages], (uint32_t)((c / stages) & 1));
+}
+
 // A wait of a kernel of a run: at most kWaitNs, and no longer than a look at the run's error word where it is set,
 // so that a run whose first wait gave up ends at once and not after a limit for each of its kernels.
 __device__ __forceinline__ bool run_wait(uint64_t *bar, uint32_t parity, const int *err) {
@@ -121,9 +128,11 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
                                          uint64_t *bars, Load load, Mma mma, Early early, Late late, Rows rows) {
    uint64_t *full = bars, *empty = full + kStages, *accFull = empty + kStages, *accEmpty = accFull + 2, *done = accEmpty + 2;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   // a run that has failed loads nothing more (read here, so that the barriers' set-up hides the latency: a failure
-   // of the kernel just before may go unseen)
-   bool ok = !(warp == kEpiWarps && lane == 0 && *reinterpret_cast<const volatile int *>(err) != 0);
+   // A run that has failed loads nothing more.  The word is read here and looked at by the load lane only, so that
+   // the set-up hides the latency (a failure of the kernel just before may go unseen).
+   int failed = 0;
+   if (warp == kEpiWarps && lane == 0) asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(failed) : "l"(err));
+   bool ok = true;
    if (threadIdx.x == 0) {
       for (int i = 0; i < bars_of<kStages>(); i++)
          mbar_init(&bars[i], &bars[i] == accEmpty || &bars[i] == accEmpty + 1 ? kEpiWarps : 1);
@@ -136,7 +145,6 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    const uint32_t tmem = *tmemBase;
    griddep_launch_dependents();
    griddep_wait();
-   int issued = 0;  // the load lane's copies
    constexpr int HALF = BN / 2, RUN = HALF < 32 ? HALF : 32;  // an epilogue warp's columns, columns per TMEM load
    auto load_run = [](uint32_t at, float *v) {
       if constexpr (RUN == 32) tmem_ld32(at, v);
@@ -145,6 +153,8 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    float acc[HALF];
    if (warp == kEpiWarps) {
       if (lane == 0) {
+         ok = failed == 0;
+         int issued = 0;
          for (int c = 0; c < chunks && ok; c++) {
             const int s = c % kStages, u = c / kStages;
             if (u > 0 && !(ok = run_wait(&empty[s], (uint32_t)((u - 1) & 1), err))) break;
@@ -152,6 +162,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
             load(c, smem + s * stageBytes, &full[s]);
             issued = c + 1;
          }
+         if (!ok) land(full, kStages, issued);  // copies in flight land before the CTA may exit
       }
    } else if (warp == kEpiWarps + 1) {
       if (lane == 0) {
@@ -206,11 +217,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    float *z = reinterpret_cast<float *>(smem);  // the stages are free: every MMA is done
    if (!good) {
       if (threadIdx.x == 0) atomicExch(err, 1);
-      // copies still in flight land before the CTA may exit, whichever role gave up: this one may have issued all
-      // of its own and gone on
-      if (warp == kEpiWarps && lane == 0)
-         for (int c = issued > kStages ? issued - kStages : 0; c < issued; c++)
-            mbar_wait(&full[c % kStages], (uint32_t)((c / kStages) & 1));
+      if (warp == kEpiWarps && lane == 0 && ok) land(full, kStages, chunks);
    } else if (warp < kEpiWarps) {
       const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * BN + (warp >> 2) * HALF;
       float *zr = z + (size_t)((warp & 3) * 32 + lane) * LZ + (warp >> 2) * HALF;

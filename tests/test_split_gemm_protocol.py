@@ -73,11 +73,11 @@ class Cta:
             (self.held if c in self.late else self.copies).append(f"full{s}")
             issued = c + 1
             yield "step"
-        if not self.drain_all and not ok:
+        if not ok:
             yield from self.drain(issued)
         yield from self.finish("load", ok)
-        if self.drain_all and not all(self.good.values()):
-            yield from self.drain(issued)
+        if self.drain_all and ok and not all(self.good.values()):
+            yield from self.drain(self.chunks)
 
     def mma(self):
         ok = True
