@@ -84,6 +84,14 @@ const char *pvgpu_last_error(void);
  * PVGPU_ERR_TIMEOUT when the wait expired (the expected result) and leaves the context usable. */
 pvgpu_status pvgpu_selftest_wait_expiry(uint64_t limitNs, long long *hostOut2, void *stream);
 
+/* The same for the gradient's GEMMs (pvgpu_lca_grad_run): two kernels in a row of one CTA whose operands never
+ * arrive, `chunks` stages of them (1..64).  The first runs its waits to the limit that the library's kernels have
+ * (0.2 s, and as much again for each of up to three copies that it would have in flight), sets the error word
+ * and writes nothing; the second finds the word set and ends at once.  Synchronous; hostOut4 receives {error word
+ * after the first, its nanoseconds, the second's, 1 if either wrote results}; returns PVGPU_ERR_TIMEOUT (the
+ * expected result). */
+pvgpu_status pvgpu_selftest_gemm_expiry(int chunks, long long *hostOut4, void *stream);
+
 /* ---- a1: active-index compaction ------------------------------------------------------
  * Replaces DataStore::updateActiveIndices (columns/DataStore.cpp:46-66), which the reference
  * runs on the host after a device->host copy.  Stable: entries of each batch element are in
@@ -415,6 +423,9 @@ pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *desc, pvgpu_lca_gr
 pvgpu_status pvgpu_lca_grad_destroy(pvgpu_lca_grad *g);
 pvgpu_status pvgpu_lca_grad_run(pvgpu_lca_grad *g, const float *w, const float *x, float *dW, double *loss,
                                 void *stream);
+/* Reads (synchronously) the error word of the last run: nonzero if a bounded device wait gave up, in which case
+ * dW and *loss are NaN. */
+pvgpu_status pvgpu_lca_grad_error_flag(const pvgpu_lca_grad *g, int *hostFlag);
 /* *emulatedFp32 = 1 when the GEMMs run as FP32 emulated on the BF16 tensor cores, 0 for plain FP32. */
 pvgpu_status pvgpu_lca_grad_info(const pvgpu_lca_grad *g, int *emulatedFp32);
 

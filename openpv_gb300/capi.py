@@ -173,6 +173,8 @@ def _declare(L):
         "pvgpu_lca_grad_destroy": (i, [vp]),
         "pvgpu_lca_grad_run": (i, [vp, vp, vp, vp, vp, vp]),
         "pvgpu_lca_grad_info": (i, [vp, C.POINTER(i)]),
+        "pvgpu_lca_grad_error_flag": (i, [vp, C.POINTER(i)]),
+        "pvgpu_selftest_gemm_expiry": (i, [i, C.POINTER(C.c_longlong), vp]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(L, name)
@@ -385,6 +387,14 @@ def selftest_wait_expiry(limit_ns, stream=None):
     return st, int(out[0]), int(out[1])
 
 
+def selftest_gemm_expiry(chunks, stream=None):
+    """(status, error word, ns of the first kernel, ns of the second, wrote) of two GEMM pipelines whose operands
+    never arrive."""
+    out = (C.c_longlong * 4)()
+    st = lib().pvgpu_selftest_gemm_expiry(int(chunks), out, _stream(stream))
+    return (st,) + tuple(int(v) for v in out)
+
+
 def tc_gemm_bf16(A, B, C, M, N, K, err, stream=None):
     check(lib().pvgpu_tc_gemm_bf16(_ptr(A), _ptr(B), _ptr(C), M, N, K, _ptr(err), _stream(stream)), "tc_gemm_bf16")
 
@@ -534,6 +544,11 @@ class LcaGrad:
     def run(self, w, x, dw, loss, stream=None):
         check(lib().pvgpu_lca_grad_run(self.h, _ptr(w), _ptr(x), _ptr(dw), _ptr(loss), _stream(stream)),
               "lca_grad_run")
+
+    def error_flag(self):
+        f = C.c_int(0)
+        check(lib().pvgpu_lca_grad_error_flag(self.h, C.byref(f)), "lca_grad_error_flag")
+        return f.value
 
     def emulated_fp32(self):
         f = C.c_int(0)

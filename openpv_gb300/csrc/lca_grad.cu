@@ -470,6 +470,19 @@ __global__ void corr_sum_kernel(int n, int splits, float om, const float *__rest
    }
 }
 
+// The pipeline without its copies: nothing ever arrives.
+__global__ void __launch_bounds__(pvgpu::split::kThreads, 1) gemm_expiry_kernel(int chunks, int *err, long long *out) {
+   using namespace pvgpu::split;
+   extern __shared__ uint8_t smem_raw[];
+   __shared__ __align__(8) uint64_t bars[bars_of<kMaxStages>()];
+   __shared__ uint32_t tmemBase;
+   const uint64_t t0 = global_ns();
+   pipeline<32, stages_of(32)>(
+         align1024(smem_raw), 3 * (kPlaneA + 32 * 128), chunks, err, &tmemBase, bars, [](int, uint8_t *, uint64_t *) {},
+         [](uint32_t, int, int, uint32_t, uint32_t) {}, [] {}, [] {}, [&](const float *, int) { out[1] = 1; });
+   if (threadIdx.x == 0) out[0] = (long long)(global_ns() - t0);
+}
+
 // ---- cuBLAS, loaded at first use --------------------------------------------------------------
 struct Blas {
    void *so = nullptr;
@@ -936,6 +949,7 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
          return pvgpu::record_message(PVGPU_ERR_LAUNCH, "lca_grad: tensor maps");
       }
       if (ok) {
+         cudaMemset(s->err, 0, sizeof(int));
          if (cudaStreamCreateWithFlags(&s->capStream, cudaStreamNonBlocking) != cudaSuccess) {
             cudaGetLastError();
             s->capStream = nullptr;
@@ -1025,6 +1039,39 @@ extern "C" pvgpu_status pvgpu_lca_grad_info(const pvgpu_lca_grad *s, int *emulat
    if (!s || !emulatedFp32) return PVGPU_ERR_BAD_ARG;
    *emulatedFp32 = s->tc || s->compute == CUBLAS_COMPUTE_32F_EMULATED_16BFX9 ? 1 : 0;
    return PVGPU_OK;
+}
+
+extern "C" pvgpu_status pvgpu_lca_grad_error_flag(const pvgpu_lca_grad *s, int *hostFlag) {
+   if (!s || !hostFlag) return PVGPU_ERR_BAD_ARG;
+   *hostFlag = 0;
+   if (s->err) PVGPU_CUDA(cudaMemcpy(hostFlag, s->err, sizeof(int), cudaMemcpyDeviceToHost), "lca_grad error flag");
+   return PVGPU_OK;
+}
+
+extern "C" pvgpu_status pvgpu_selftest_gemm_expiry(int chunks, long long *hostOut4, void *stream) {
+   if (!hostOut4 || chunks < 1 || chunks > 64) return PVGPU_ERR_BAD_ARG;
+   cudaStream_t s = pvgpu::as_stream(stream);
+   constexpr size_t kWords = 8;  // error word, then each kernel's time and whether it wrote
+   long long host[kWords] = {}, *d = nullptr;
+   PVGPU_CUDA(cudaFuncSetAttribute(gemm_expiry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(32)),
+              "selftest_gemm_expiry");
+   PVGPU_CUDA(cudaMallocAsync(&d, sizeof(host), s), "selftest_gemm_expiry");
+   cudaError_t e = cudaMemsetAsync(d, 0, sizeof(host), s);
+   for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+      gemm_expiry_kernel<<<1, pvgpu::split::kThreads, gemm_smem(32), s>>>(chunks, reinterpret_cast<int *>(d), d + 2 + 2 * k);
+      e = cudaGetLastError();
+      if (e == cudaSuccess && k == 0) e = cudaMemcpyAsync(host + 6, d, sizeof(int), cudaMemcpyDeviceToHost, s);
+   }
+   if (e == cudaSuccess) e = cudaMemcpyAsync(host, d, 6 * sizeof(long long), cudaMemcpyDeviceToHost, s);
+   const cudaError_t f = cudaFreeAsync(d, s);
+   if (e == cudaSuccess) e = f;
+   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+   if (e != cudaSuccess) return pvgpu::record_cuda_error(e, "selftest_gemm_expiry");
+   hostOut4[0] = (int)host[6];
+   hostOut4[1] = host[2];
+   hostOut4[2] = host[4];
+   hostOut4[3] = host[3] || host[5];
+   return hostOut4[0] ? PVGPU_ERR_TIMEOUT : PVGPU_OK;
 }
 
 extern "C" pvgpu_status pvgpu_lca_grad_run(pvgpu_lca_grad *s, const float *W, const float *x, float *dW,
