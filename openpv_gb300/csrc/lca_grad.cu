@@ -341,17 +341,20 @@ __global__ void split_activity_kernel(int64_t n8, float vt, const float *__restr
 // fold_kernel), staged in shared memory, then every position's patch written as planes times signOut.
 // Neighbouring bands gather the P - S rows they share twice, from L2; in exchange the image and the
 // FP32 im2col never go to memory and the pass is one launch (23 us for the two before, 9 now).
-// SS, PP, CC: the geometry as constants, or 0.
+// SS, PP, CC: the geometry as constants, or 0.  Any other geometry takes xPer positions of a row at a time: its
+// gather is a chain of loads per pixel, so where bands are few and patches large a row is divided (3 x 56x76x3 ->
+// 14x19x8, 16x16 patches, 16 steps: 2.49 ms with whole rows, now 1.65; the library path 1.25).
 constexpr int kMaxBandRows = 2, kFoldThreads = 384;
 template <int SS, int PP, int CC>
-__global__ void __launch_bounds__(kFoldThreads, 2) fold_im2col_kernel(Geo g, int bandRows, const float *__restrict__ D, const float *__restrict__ x,
-                                                          float signImg, float signOut, bf16 *__restrict__ out,
-                                                          size_t plane) {
+__global__ void __launch_bounds__(kFoldThreads, 2) fold_im2col_kernel(Geo g, int bandRows, int xPer, const float *__restrict__ D,
+                                                                      const float *__restrict__ x, float signImg, float signOut,
+                                                                      bf16 *__restrict__ out, size_t plane) {
    extern __shared__ __align__(16) float win[];
    const int S = SS ? SS : g.S, P = PP ? PP : g.P, C = CC ? CC : g.C, E = (P - S) / 2, PC = P * C, KP = P * PC;
    const int bands = (g.vy + bandRows - 1) / bandRows;
    const int b = blockIdx.x / bands, y0 = (blockIdx.x % bands) * bandRows, rows = min(bandRows, g.vy - y0);
-   const int WP = ((g.inx + 2 * E) * C + 3) & ~3, WR = S * (rows - 1) + P;
+   const int x0 = SS ? 0 : blockIdx.y * xPer, xn = SS ? g.vx : min(xPer, g.vx - x0);  // positions of a row
+   const int WP = ((SS ? g.inx + 2 * E : S * (xn - 1) + P) * C + 3) & ~3, WR = S * (rows - 1) + P;
    griddep_launch_dependents();
    griddep_wait();
    const float *Db = D + (size_t)b * g.Np * KP;
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) fold_im2col_kernel(Geo g, int
    } else {
       for (int i = threadIdx.x; i < WR * WP; i += blockDim.x) {
          const int yy = i / WP, col = i - yy * WP;
-         const int iy = S * y0 - E + yy, j = col - E * C;
+         const int iy = S * y0 - E + yy, j = col + (S * x0 - E) * C;
          float r = 0.0f;
          if (iy >= 0 && iy < g.iny && j >= 0 && j < g.inx * C) {
             const int ix = j / C, c = j - ix * C;
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) fold_im2col_kernel(Geo g, int
             float s = 0.0f;
             for (int py = pyLo; py <= pyHi; py++) {
                const float *d = Db + ((size_t)py * g.vx + pxLo) * KP + ((iy + E - S * py) * P + ix + E - S * pxLo) * C + c;
-   #pragma unroll 4
+#pragma unroll 4
                for (int px = pxLo; px <= pxHi; px++, d += KP - S * C) s += __ldg(d);
             }
             r = (x ? x[((size_t)b * g.iny + iy) * g.inx * C + j] : 0.0f) + signImg * s;
@@ -424,10 +427,10 @@ __global__ void __launch_bounds__(kFoldThreads, 2) fold_im2col_kernel(Geo g, int
       }
    }
    __syncthreads();
-   const int k8 = KP / 8, items = rows * g.vx * k8;
-   bf16 *o = out + ((size_t)b * g.Np + (size_t)y0 * g.vx) * KP;
+   const int k8 = KP / 8, items = rows * xn * k8;
+   bf16 *o = out + ((size_t)b * g.Np + (size_t)y0 * g.vx + x0) * KP;
    for (int i = threadIdx.x; i < items; i += blockDim.x) {
-      const int p = i / k8, k = (i - p * k8) * 8, yl = p / g.vx, xl = p - yl * g.vx;
+      const int p = i / k8, k = (i - p * k8) * 8, yl = p / xn, xl = p - yl * xn;
       const float *w = win + (S * yl) * WP + S * xl * C;
       int ky = k / PC, rem = k - ky * PC;
       float v[8];
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) fold_im2col_kernel(Geo g, int
             }
          }
       }
-      split_store8(v, o + (size_t)p * KP + k, plane);
+      split_store8(v, o + (size_t)(yl * g.vx + xl) * KP + k, plane);
    }
 }
 
@@ -553,7 +556,7 @@ struct pvgpu_lca_grad {
    size_t planeA = 0, planeR = 0;  // values of one plane of pA (K slots) and of pR (K + 1 slots)
    bf16 *ckLo = nullptr, *vLo = nullptr, *sVLo = nullptr;  // the low parts of ck, V[0] and sV
    float *P = nullptr;             // partial correlations
-   int splits = 0, bn = 128, bandRows = kMaxBandRows;
+   int splits = 0, bn = 128, bandRows = kMaxBandRows, xPer = 1;
    int *err = nullptr;
    CUtensorMap mA, mR, mG, mGD, mW, mWT;        // operands of the GEMMs (W's as B)
    CUtensorMap cA, cR, cG, cGD;                 // the same planes as operands of the correlations
@@ -699,8 +702,8 @@ constexpr size_t kCorrSmem = 2 * 6 * (size_t)pvgpu::split::kPlaneA + 1024;
 // the kernel, not to a handle, so it is set to the bound and never to one handle's size.
 constexpr size_t kBandSmem = 200 * 1024;
 
-size_t band_smem(const Geo &g) {
-   return sizeof(float) * (size_t)(g.S * (kMaxBandRows - 1) + g.P) * (((g.inx + 2 * g.E) * g.C + 3) & ~3);
+size_t band_smem(const Geo &g, int xPer) {
+   return sizeof(float) * (size_t)(g.S * (kMaxBandRows - 1) + g.P) * (((g.S * (xPer - 1) + g.P) * g.C + 3) & ~3);
 }
 
 template <typename Epi>
@@ -723,6 +726,10 @@ bool gemm_attrs() {
           cudaFuncSetAttribute(gemm_kernel<32, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(32)) == cudaSuccess;
 }
 
+bool special_geometry(const Geo &g) {
+   return (g.S == 4 && g.P == 16 && g.C == 1) || (g.S == 2 && g.P == 8 && (g.C == 1 || g.C == 3));
+}
+
 template <typename Fn>
 auto with_geometry(const Geo &g, Fn &&fn) {
    if (g.S == 4 && g.P == 16 && g.C == 1) return fn(fold_im2col_kernel<4, 16, 1>);
@@ -734,9 +741,10 @@ auto with_geometry(const Geo &g, Fn &&fn) {
 pvgpu_status fold_im2col(pvgpu_lca_grad *s, cudaStream_t st, const float *x, float signImg, float signOut, bf16 *out,
                          size_t plane) {
    const Geo &g = s->g;
-   const dim3 grid((unsigned)(g.nb * ((g.vy + s->bandRows - 1) / s->bandRows)));
+   const dim3 grid((unsigned)(g.nb * ((g.vy + s->bandRows - 1) / s->bandRows)), (g.vx + s->xPer - 1) / s->xPer);
    return with_geometry(g, [&](auto kernel) {
-      return launch_pdl(kernel, grid, kFoldThreads, band_smem(g), st, g, s->bandRows, (const float *)s->D, x, signImg, signOut, out, plane);
+      return launch_pdl(kernel, grid, kFoldThreads, band_smem(g, s->xPer), st, g, s->bandRows, s->xPer, (const float *)s->D, x, signImg,
+                        signOut, out, plane);
    });
 }
 
@@ -900,7 +908,7 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
    // shared memory
    bool noRoom = false;
    s->tc = ok && d->VThresh >= 0.0f && g.F % 8 == 0 && g.KP % 8 == 0 && g.M <= 0x7fffff00LL && (g.M + 127) / 128 <= 65535 &&
-           (int64_t)g.nb * g.vy <= 0x7fffffff && band_smem(g) <= kBandSmem &&
+           (int64_t)g.nb * g.vy <= 0x7fffffff && band_smem(g, g.vx) <= kBandSmem &&
            (size_t)g.F * g.KP <= 0x7fffffff && pvgpu::encode_tiled_fn() != nullptr;
    if (s->tc) {
       auto planes = [&](bf16 **p, size_t n) { alloc(reinterpret_cast<void **>(p), 3 * n * sizeof(bf16)); };
@@ -931,6 +939,16 @@ extern "C" pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *d, pvgp
       s->bn = 128;
       for (int bn = 64; bn >= 32 && mTiles * ((n + bn - 1) / bn) <= sms; bn /= 2) s->bn = bn;
       s->bandRows = (int64_t)g.nb * ((g.vy + 1) / 2) < sms / 2 ? 1 : 2;
+      // positions of a row per CTA: whole rows, but where these leave half of the SMs idle and a thread more than
+      // ten loads of the gather in a row, as few (two at least) as give every SM two CTAs.  Over 230 geometries:
+      // 5 to 25 % of a run there; elsewhere the overlap of the parts' windows costs 2 to 18 %.
+      s->xPer = g.vx;
+      const int64_t bands = (int64_t)g.nb * ((g.vy + s->bandRows - 1) / s->bandRows);
+      const double loads = (double)band_smem(g, g.vx) / 4 / kFoldThreads * (g.P / S) * (g.P / S);
+      if (!special_geometry(g) && bands < sms / 2 && loads >= 10) {
+         const int64_t parts = std::min<int64_t>((2 * sms + bands - 1) / bands, (g.vx + 1) / 2);
+         s->xPer = (int)((g.vx + parts - 1) / parts);
+      }
       using pvgpu::split::make_map;
       const uint64_t M = (uint64_t)g.M, F = g.F, KP = g.KP;
       if (ok && !(make_map(&s->mA, s->pA, s->planeA, K + 1, M, F, 128) && make_map(&s->mR, s->pR, s->planeR, K + 1, M, KP, 128) &&
