@@ -1682,7 +1682,7 @@ __global__ void v_layout_kernel(LcaGeom g, const float *__restrict__ src, float 
 // The SIMT FP32 form lives in lca_solver_fp32.cu and shares LcaGeom through this hook.
 namespace pvgpu {
 pvgpu_status lca_fp32_step(int S, int P, int C, const LcaGeom &g, const float *x, const float *W32, const float *Wt32,
-                           float *D, float *rpad, float *V, float *A32, cudaStream_t s, cudaEvent_t mid);
+                           float *D, int imagesPerD, float *rpad, float *V, float *A32, cudaStream_t s, cudaEvent_t mid);
 }
 
 // Images [img0, img0 + g.nb) of the batch as a batch of their own: the geometry and the tensor
@@ -1710,7 +1710,8 @@ struct pvgpu_lca_solver {
    float *bands = nullptr;  // kernel F's bands, two buffers (a step reads one and writes the other)
    float *xpad = nullptr;   // x in the padded layout (kernel F)
    size_t bandsPerBuf = 0;  // floats in one band buffer (sized for 128-feature tiles)
-   float *D32 = nullptr;    // the FP32 form's A . W [nbatch * positions][KP]: its own, or the bands' memory
+   float *D32 = nullptr;    // the FP32 form's A . W [imagesPerD * positions][KP]: its own, or the bands' memory
+   int imagesPerD = 0;
    bool ownD32 = false;
    bool padValid = false;  // rpad holds the residual of the last step
    bool weightsSet = false;
@@ -2316,15 +2317,23 @@ extern "C" pvgpu_status pvgpu_lca_solver_create(const pvgpu_lca_solver_desc *d, 
          std::memset(&s->fplan, 0, sizeof(s->fplan));
       }
    }
-   // the FP32 form's reconstruction GEMM output lives in the bands, which hold nothing between runs,
-   // where they are large enough
-   const size_t nD = (size_t)g.nb * Npos * KP;
-   if (s->bands && 2 * s->bandsPerBuf >= nD) s->D32 = s->bands;
-   else if (cudaMalloc(&s->D32, nD * 4) == cudaSuccess) s->ownD32 = true;
-   else {
+   // The FP32 form's reconstruction GEMM output lives in the bands, which hold nothing between runs, where they are
+   // large enough; else in 64 MB or less (its share of L2; 340 images of 32x32x3), for that many images at a time.
+   const size_t perImage = (size_t)Npos * KP;
+   if (s->bands && 2 * s->bandsPerBuf >= g.nb * perImage) {
+      s->D32 = s->bands;
+      s->imagesPerD = g.nb;
+   } else {
+      for (size_t n = std::min<size_t>(g.nb, std::max<size_t>(1, (64u << 20) / 4 / perImage)); n > 0 && !s->D32; n /= 2)
+         if (cudaMalloc(&s->D32, n * perImage * 4) == cudaSuccess) s->imagesPerD = (int)n;
+         else s->D32 = nullptr;
+      if (!s->D32) {
+         cudaGetLastError();
+         free_solver(s);
+         return PVGPU_ERR_OOM;
+      }
       cudaGetLastError();
-      free_solver(s);
-      return PVGPU_ERR_OOM;
+      s->ownD32 = true;
    }
    s->rplan = make_recon_plan(g, S, P, C, false, g_num_sms);
    s->rplanX3 = make_recon_plan(g, S, P, C, true, g_num_sms);
@@ -2414,7 +2423,8 @@ extern "C" pvgpu_status pvgpu_lca_solver_run(pvgpu_lca_solver *s, const float *x
       for (int t = 0; t < numSteps; t++) {
          const bool rec = s->profiling && s->evNext + 3 <= s->ev.size();
          if (rec) cudaEventRecord(s->ev[s->evNext], st);
-         pvgpu_status r = pvgpu::lca_fp32_step(s->S, s->P, s->C, s->g, x, s->W32, s->Wt32, s->D32, s->rpad, s->V, s->A32,
+         pvgpu_status r = pvgpu::lca_fp32_step(s->S, s->P, s->C, s->g, x, s->W32, s->Wt32, s->D32,
+                                               s->imagesPerD, s->rpad, s->V, s->A32,
                                                st, rec ? s->ev[s->evNext + 1] : nullptr);
          if (r != PVGPU_OK) return r;
          if (rec) {

@@ -115,18 +115,23 @@ __global__ void __launch_bounds__(128) fold_residual_kernel(LcaGeom g, int rowsP
 }
 
 template <int S, int P, int C>
-pvgpu_status step(const LcaGeom &g, const float *x, const float *W32, const float *Wt32, float *D, float *rpad, float *V,
-                  float *A32, cudaStream_t st, cudaEvent_t mid) {
+pvgpu_status step(const LcaGeom &g, const float *x, const float *W32, const float *Wt32, float *D, int imagesPerD, float *rpad,
+                  float *V, float *A32, cudaStream_t st, cudaEvent_t mid) {
    constexpr int KP = P * P * C, E = (P - S) / 2;
    const int64_t M = (int64_t)g.nb * g.Npos;
    const int RP = ((g.inNx + 2 * E) * C + 3) & ~3, rowsPad = g.inNy + 2 * E;
+   const size_t nPix = (size_t)g.inNx * g.inNy * C;
    if (M > 0x7fffffff) return PVGPU_ERR_UNSUPPORTED_SHAPE;
-   const ReconProblem rp = {M, KP, g.F, g.F, 0, A32, Wt32, D};
-   pvgpu_status r = pvgpu::fp32_gemm::run<4>(rp, 1, st, "lca32 recon");
-   if (r != PVGPU_OK) return r;
-   const dim3 fg(g.nb, rowsPad, (RP + 127) / 128);
-   fold_residual_kernel<S, P, C><<<fg, 128, 0, st>>>(g, rowsPad, RP, x, D, rpad);
-   PVGPU_CHECK_LAUNCH("lca32 fold");
+   for (int b0 = 0; b0 < g.nb; b0 += imagesPerD) {  // as many images as D holds
+      LcaGeom part = g;
+      part.nb = std::min(imagesPerD, g.nb - b0);
+      const ReconProblem rp = {(int64_t)part.nb * g.Npos, KP, g.F, g.F, 0, A32 + (size_t)b0 * g.Npos * g.F, Wt32, D};
+      const pvgpu_status r = pvgpu::fp32_gemm::run<4>(rp, 1, st, "lca32 recon");
+      if (r != PVGPU_OK) return r;
+      const dim3 fg(part.nb, rowsPad, (RP + 127) / 128);
+      fold_residual_kernel<S, P, C><<<fg, 128, 0, st>>>(part, rowsPad, RP, x + b0 * nPix, D, rpad + (size_t)b0 * rowsPad * RP);
+      PVGPU_CHECK_LAUNCH("lca32 fold");
+   }
    if (mid) cudaEventRecord(mid, st);
    // windows start at multiples of S * C floats, their rows of P * C values RP (a multiple of 4) apart
    constexpr int VW = S * C % 4 == 0 ? 4 : 2;
@@ -142,11 +147,13 @@ pvgpu_status step(const LcaGeom &g, const float *x, const float *W32, const floa
 
 namespace pvgpu {
 
+// D: room for the reconstruction GEMM of imagesPerD images
 pvgpu_status lca_fp32_step(int S, int P, int C, const LcaGeom &g, const float *x, const float *W32, const float *Wt32,
-                           float *D, float *rpad, float *V, float *A32, cudaStream_t st, cudaEvent_t mid) {
-   if (S == 2 && P == 8 && C == 1) return step<2, 8, 1>(g, x, W32, Wt32, D, rpad, V, A32, st, mid);
-   if (S == 2 && P == 8 && C == 3) return step<2, 8, 3>(g, x, W32, Wt32, D, rpad, V, A32, st, mid);
-   if (S == 4 && P == 16 && C == 1) return step<4, 16, 1>(g, x, W32, Wt32, D, rpad, V, A32, st, mid);
+                           float *D, int imagesPerD, float *rpad, float *V, float *A32, cudaStream_t st,
+                           cudaEvent_t mid) {
+   if (S == 2 && P == 8 && C == 1) return step<2, 8, 1>(g, x, W32, Wt32, D, imagesPerD, rpad, V, A32, st, mid);
+   if (S == 2 && P == 8 && C == 3) return step<2, 8, 3>(g, x, W32, Wt32, D, imagesPerD, rpad, V, A32, st, mid);
+   if (S == 4 && P == 16 && C == 1) return step<4, 16, 1>(g, x, W32, Wt32, D, imagesPerD, rpad, V, A32, st, mid);
    return PVGPU_ERR_UNSUPPORTED_SHAPE;
 }
 
