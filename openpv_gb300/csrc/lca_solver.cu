@@ -1545,11 +1545,11 @@ __global__ void pad_x_kernel(LcaGeom g, int C, int E, int rowsPad, int RP, const
 // Probe energy: l2Coeff * sum r^2 + costCoeff * sum cost(T(V)), per image, FP64
 // (ColumnEnergyProbe.cpp:60-70 over L2NormProbe and L1NormLCAProbe / FirmThresholdCostFnLCAProbe)
 // -------------------------------------------------------------------------------------------
-// The residual comes from the padded residual of kernel R (zero border) when rpad is given,
-// else (no timestep since the reset) it is x.
+// The residual comes from the padded residual of kernel R (zero border) when rpad is given, from x and
+// the reconstruction of the FP32 form's last step when rec is, else (no timestep since the reset) it is x.
 __global__ void __launch_bounds__(256) energy_kernel(LcaGeom g, int C, const float *__restrict__ x,
                                                      const float *__restrict__ rpad, int padPerImage,
-                                                     const float *__restrict__ V, double l2Coeff, int costKind,
+                                                     const float *__restrict__ rec, const float *__restrict__ V, double l2Coeff, int costKind,
                                                      double cp0, double cp1, double costCoeff,
                                                      double *__restrict__ out) {
    const int b = blockIdx.x;
@@ -1563,7 +1563,8 @@ __global__ void __launch_bounds__(256) energy_kernel(LcaGeom g, int C, const flo
       }
    } else {
       for (int i = threadIdx.x; i < nPix; i += 256) {
-         const double r = (double)x[(size_t)b * nPix + i];
+         const size_t at = (size_t)b * nPix + i;
+         const double r = (double)(rec ? __fadd_rn(x[at], -rec[at]) : x[at]);
          l2 += r * r;
       }
    }
@@ -1682,7 +1683,8 @@ __global__ void v_layout_kernel(LcaGeom g, const float *__restrict__ src, float 
 // The SIMT FP32 form lives in lca_solver_fp32.cu and shares LcaGeom through this hook.
 namespace pvgpu {
 pvgpu_status lca_fp32_step(int S, int P, int C, const LcaGeom &g, const float *x, const float *W32, const float *Wt32,
-                           float *D, int imagesPerD, float *rpad, float *V, float *A32, cudaStream_t s, cudaEvent_t mid);
+                           float *D, int imagesPerD, float *rpad, float *rec, float *V, float *A32, cudaStream_t s,
+                           cudaEvent_t mid);
 }
 
 // Images [img0, img0 + g.nb) of the batch as a batch of their own: the geometry and the tensor
@@ -1713,7 +1715,9 @@ struct pvgpu_lca_solver {
    float *D32 = nullptr;    // the FP32 form's A . W [imagesPerD * positions][KP]: its own, or the bands' memory
    int imagesPerD = 0;
    bool ownD32 = false;
-   bool padValid = false;  // rpad holds the residual of the last step
+   float *rec = nullptr;    // the reconstruction of the FP32 form's last step [nbatch][pixels]
+   bool padValid = false;   // rpad holds the residual of the last step, which the BF16 form took
+   bool recValid = false;   // rec holds the reconstruction of the last step, which the FP32 form took
    bool weightsSet = false;
    // optional per-kernel timing: events before kernel R, between R and P, after P
    std::vector<cudaEvent_t> ev;
@@ -2140,7 +2144,7 @@ void free_solver(pvgpu_lca_solver *s) {
    if (s->capStream2) cudaStreamDestroy(s->capStream2);
    if (s->forkEv) cudaEventDestroy(s->forkEv);
    if (s->joinEv) cudaEventDestroy(s->joinEv);
-   void *ptrs[] = {s->V,   s->ownD32 ? s->D32 : nullptr, s->rpad, s->A32, s->W32, s->Wt32,  s->A,
+   void *ptrs[] = {s->V,   s->ownD32 ? s->D32 : nullptr, s->rec, s->rpad, s->A32, s->W32, s->Wt32,  s->A,
                    s->Alo, s->W,        s->Wlo,  s->Wt,  s->Wtlo, s->bands, s->xpad, s->err};
    for (void *p : ptrs)
       if (p) cudaFree(p);
@@ -2247,7 +2251,8 @@ extern "C" pvgpu_status pvgpu_lca_solver_create(const pvgpu_lca_solver_desc *d, 
              cudaMalloc(&s->Wlo, nW * 2) == cudaSuccess && cudaMalloc(&s->Wt, nW * 2) == cudaSuccess &&
              cudaMalloc(&s->Wtlo, nW * 2) == cudaSuccess && cudaMalloc(&s->W32, nW * 4) == cudaSuccess &&
              cudaMalloc(&s->Wt32, nW * 4) == cudaSuccess && cudaMalloc(&s->err, sizeof(int)) == cudaSuccess &&
-             cudaMalloc(&s->rpad, nPad * 4) == cudaSuccess;
+             cudaMalloc(&s->rpad, nPad * 4) == cudaSuccess &&
+             cudaMalloc(&s->rec, (size_t)g.nb * d->inNx * d->inNy * C * 4) == cudaSuccess;
    if (!ok) {
       cudaGetLastError();
       free_solver(s);
@@ -2410,7 +2415,7 @@ extern "C" pvgpu_status pvgpu_lca_solver_reset(pvgpu_lca_solver *s, const float 
    PVGPU_CHECK_LAUNCH("lca reset");
    PVGPU_CUDA(cudaMemsetAsync(s->err, 0, sizeof(int), st), "lca reset");
    s->stepsRun = 0;
-   s->padValid = false;
+   s->padValid = s->recValid = false;
    return PVGPU_OK;
 }
 
@@ -2424,7 +2429,7 @@ extern "C" pvgpu_status pvgpu_lca_solver_run(pvgpu_lca_solver *s, const float *x
          const bool rec = s->profiling && s->evNext + 3 <= s->ev.size();
          if (rec) cudaEventRecord(s->ev[s->evNext], st);
          pvgpu_status r = pvgpu::lca_fp32_step(s->S, s->P, s->C, s->g, x, s->W32, s->Wt32, s->D32,
-                                               s->imagesPerD, s->rpad, s->V, s->A32,
+                                               s->imagesPerD, s->rpad, t + 1 == numSteps ? s->rec : nullptr, s->V, s->A32,
                                                st, rec ? s->ev[s->evNext + 1] : nullptr);
          if (r != PVGPU_OK) return r;
          if (rec) {
@@ -2433,7 +2438,10 @@ extern "C" pvgpu_status pvgpu_lca_solver_run(pvgpu_lca_solver *s, const float *x
          }
       }
       s->stepsRun += numSteps;
-      if (numSteps > 0) s->padValid = true;
+      if (numSteps > 0) {
+         s->padValid = false;
+         s->recValid = true;
+      }
       return PVGPU_OK;
    }
    if (precision != PVGPU_LCA_BF16) return PVGPU_ERR_BAD_ARG;
@@ -2485,7 +2493,10 @@ extern "C" pvgpu_status pvgpu_lca_solver_run(pvgpu_lca_solver *s, const float *x
       if (r != PVGPU_OK) return r;
    }
    s->stepsRun += numSteps;
-   if (numSteps > 0) s->padValid = true;
+   if (numSteps > 0) {
+      s->padValid = true;
+      s->recValid = false;
+   }
    return PVGPU_OK;
 }
 
@@ -2495,7 +2506,7 @@ extern "C" pvgpu_status pvgpu_lca_solver_energy(pvgpu_lca_solver *s, const float
    if (!s || !x || !energy || (costKind != 1 && costKind != 2)) return PVGPU_ERR_BAD_ARG;
    energy_kernel<<<s->g.nb, 256, 0, pvgpu::as_stream(stream)>>>(s->g, s->C, x,
                                                                 s->padValid ? s->rpad : nullptr, s->rplan.rowsPad * s->rplan.RP,
-                                                                s->V, l2Coeff, costKind, costThresh, costWidth,
+                                                                s->recValid ? s->rec : nullptr, s->V, l2Coeff, costKind, costThresh, costWidth,
                                                                 costCoeff, energy);
    PVGPU_CHECK_LAUNCH("lca energy");
    return PVGPU_OK;

@@ -82,7 +82,7 @@ template <int S, int P, int C>
 __global__ void __launch_bounds__(128) fold_residual_kernel(LcaGeom g, int rowsPad, int RP,
                                                                  const float *__restrict__ x,
                                                                  const float *__restrict__ D,
-                                                                 float *__restrict__ rpad) {
+                                                                 float *__restrict__ rpad, float *__restrict__ recOut) {
    constexpr int KP = P * P * C, E = (P - S) / 2, Q = P / S;
    const int yp = blockIdx.y, b = blockIdx.x;
    const int col = blockIdx.z * blockDim.x + threadIdx.x;
@@ -109,14 +109,16 @@ __global__ void __launch_bounds__(128) fold_residual_kernel(LcaGeom g, int rowsP
       for (int qy = 0; qy < Q; qy++)
 #pragma unroll
          for (int qx = 0; qx < Q; qx++) rec += t[qy][qx];
-      r = x[((size_t)b * g.inNy + iy) * g.inNx * C + j] - rec;
+      const size_t at = ((size_t)b * g.inNy + iy) * g.inNx * C + j;
+      r = x[at] - rec;
+      if (recOut) recOut[at] = rec;
    }
    rpad[((size_t)b * rowsPad + yp) * RP + col] = r;
 }
 
 template <int S, int P, int C>
 pvgpu_status step(const LcaGeom &g, const float *x, const float *W32, const float *Wt32, float *D, int imagesPerD, float *rpad,
-                  float *V, float *A32, cudaStream_t st, cudaEvent_t mid) {
+                  float *rec, float *V, float *A32, cudaStream_t st, cudaEvent_t mid) {
    constexpr int KP = P * P * C, E = (P - S) / 2;
    const int64_t M = (int64_t)g.nb * g.Npos;
    const int RP = ((g.inNx + 2 * E) * C + 3) & ~3, rowsPad = g.inNy + 2 * E;
@@ -129,7 +131,8 @@ pvgpu_status step(const LcaGeom &g, const float *x, const float *W32, const floa
       const pvgpu_status r = pvgpu::fp32_gemm::run<4>(rp, 1, st, "lca32 recon");
       if (r != PVGPU_OK) return r;
       const dim3 fg(part.nb, rowsPad, (RP + 127) / 128);
-      fold_residual_kernel<S, P, C><<<fg, 128, 0, st>>>(part, rowsPad, RP, x + b0 * nPix, D, rpad + (size_t)b0 * rowsPad * RP);
+      fold_residual_kernel<S, P, C><<<fg, 128, 0, st>>>(part, rowsPad, RP, x + b0 * nPix, D, rpad + (size_t)b0 * rowsPad * RP,
+                                                       rec ? rec + b0 * nPix : nullptr);
       PVGPU_CHECK_LAUNCH("lca32 fold");
    }
    if (mid) cudaEventRecord(mid, st);
@@ -147,13 +150,14 @@ pvgpu_status step(const LcaGeom &g, const float *x, const float *W32, const floa
 
 namespace pvgpu {
 
-// D: room for the reconstruction GEMM of imagesPerD images
+// D: room for the reconstruction GEMM of imagesPerD images; rec: the step's reconstruction W^T a (what the energy
+// probe subtracts from the image it is given), or null
 pvgpu_status lca_fp32_step(int S, int P, int C, const LcaGeom &g, const float *x, const float *W32, const float *Wt32,
-                           float *D, int imagesPerD, float *rpad, float *V, float *A32, cudaStream_t st,
+                           float *D, int imagesPerD, float *rpad, float *rec, float *V, float *A32, cudaStream_t st,
                            cudaEvent_t mid) {
-   if (S == 2 && P == 8 && C == 1) return step<2, 8, 1>(g, x, W32, Wt32, D, imagesPerD, rpad, V, A32, st, mid);
-   if (S == 2 && P == 8 && C == 3) return step<2, 8, 3>(g, x, W32, Wt32, D, imagesPerD, rpad, V, A32, st, mid);
-   if (S == 4 && P == 16 && C == 1) return step<4, 16, 1>(g, x, W32, Wt32, D, imagesPerD, rpad, V, A32, st, mid);
+   if (S == 2 && P == 8 && C == 1) return step<2, 8, 1>(g, x, W32, Wt32, D, imagesPerD, rpad, rec, V, A32, st, mid);
+   if (S == 2 && P == 8 && C == 3) return step<2, 8, 3>(g, x, W32, Wt32, D, imagesPerD, rpad, rec, V, A32, st, mid);
+   if (S == 4 && P == 16 && C == 1) return step<4, 16, 1>(g, x, W32, Wt32, D, imagesPerD, rpad, rec, V, A32, st, mid);
    return PVGPU_ERR_UNSUPPORTED_SHAPE;
 }
 
