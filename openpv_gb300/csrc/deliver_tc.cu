@@ -77,6 +77,11 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
    return reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
 }
 
+// The last of `sent` copies through a ring of `slots` barriers land (out of line: only a failing run calls it).
+__device__ __noinline__ void land(uint64_t *full, int slots, uint32_t sent) {
+   for (uint32_t c = sent > (uint32_t)slots ? sent - slots : 0; c < sent; c++) mbar_wait(&full[c % slots], (c / slots) & 1);
+}
+
 // R = target rows per unit (g.R); NCH = R * NT / 32: 32-column chunks of the result, summed in
 // registers by the epilogue (a chain buffer holds 2 * NCH chunks: hi-weight and lo-weight
 // columns).  R is a template parameter so that the 8R MMAs of one weight tile issue as one
@@ -92,6 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
          bFull[kMaxNB], bEmpty[kMaxNB], chainFull[2], chainEmpty[2], mmaDone;
    __shared__ uint32_t tmemBase;
    __shared__ volatile int abortFlag;
+   __shared__ uint32_t sentA, sentB;  // raw rows and weight tiles that the producer has issued
 
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    const uint32_t bBytes = (uint32_t)g.NT * 128;  // one TF32 weight tile (NT rows x 32)
@@ -188,11 +194,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
                }
             }
          }
-         // copies still in flight must land before the CTA may exit
-         if (!ok) {
-            for (uint32_t c = ca > (uint32_t)g.NR ? ca - g.NR : 0; c < ca; c++) mbar_wait(&rawFull[c % g.NR], (c / g.NR) & 1);
-            for (uint32_t c = cb > (uint32_t)g.NB ? cb - g.NB : 0; c < cb; c++) mbar_wait(&bFull[c % g.NB], (c / g.NB) & 1);
-         }
+         sentA = ca;
+         sentB = cb;
       }
    } else if (warp == 1) {
       // ================================ MMA issuer ================================
@@ -404,7 +407,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
       }
    }
    __syncthreads();
-   if (tid == 0 && abortFlag) atomicExch(err, 1);
+   if (tid == 0 && abortFlag) {
+      atomicExch(err, 1);
+      // copies still in flight must land before the CTA may exit, whichever role gave up: the producer may have
+      // issued all of its own by then
+      land(rawFull, g.NR, sentA);
+      land(bFull, g.NB, sentB);
+   }
    tc_fence_before();
    __syncthreads();
    if (warp == 1) tmem_dealloc(tmem, g.tmemCols);

@@ -7,25 +7,20 @@ a barrier more than one phase away.  With copies that are late, every wait is bo
 the limit passes and the waits open at that moment give up.  Whatever is late then, the CTA must not exit with a
 copy in flight, unless the wait for that very copy ran out as well.  And a run of many such kernels, of which one
 has given up, must end without a limit for each of the others."""
-import random
-
 import pytest
+
+from tests.mbar_sim import Cta
 
 EPI = 8
 
 
-class Cta:
-    """One CTA.  late: copies (chunk numbers) that land only after `after` limits have passed.  failed: the run's
-    error word on entry, which the load lane reads first and the other waits when they are not over at once."""
+class Pipeline(Cta):
+    """failed: the run's error word on entry, which the load lane reads first and the other waits when they are not
+    over at once."""
 
     def __init__(self, chunks, stages, seed, late=(), after=1, drain_all=True, failed=False):
-        self.chunks, self.stages, self.rnd = chunks, stages, random.Random(seed)
-        self.late, self.after, self.drain_all = set(late), after, drain_all
-        self.failed = failed
-        self.limits = 0  # limits that passed
-        self.gen = 0
-        self.count, self.pending, self.done = {}, {}, {}
-        self.copies, self.held, self.commits, self.aliased = [], [], [], []
+        super().__init__(seed, late, after)
+        self.chunks, self.stages, self.drain_all, self.failed = chunks, stages, drain_all, failed
         for i in range(stages):
             self.mk(f"full{i}")
             self.mk(f"empty{i}")
@@ -34,34 +29,15 @@ class Cta:
             self.mk(f"accEmpty{i}", EPI)
         self.mk("done")
         self.good = {}
-        self.landing_given_up = 0  # waits for a copy in flight that ran out in the drain
-
-    def mk(self, name, n=1):
-        self.count[name], self.pending[name], self.done[name] = n, 0, 0
-
-    def arrive(self, name):
-        self.pending[name] += 1
-        if self.pending[name] == self.count[name]:
-            self.pending[name] = 0
-            self.done[name] += 1
 
     def wait(self, name, k):
-        """Phase k of a barrier; False when the limit passes first."""
-        gen = self.gen
-        while True:
-            d = self.done[name]
-            if not k <= d <= k + 1:
-                self.aliased.append((name, k, d))
-            if (d & 1) != (k & 1):
-                return True
-            if self.gen != gen or (self.failed and name != "done"):
-                return False
-            yield "blocked"
+        if self.failed and name != "done":
+            yield "step"
+            return self.test(name, k)
+        return (yield from super().wait(name, k))
 
     def drain(self, issued):
-        for c in range(max(0, issued - self.stages), issued):
-            if not (yield from self.wait(f"full{c % self.stages}", c // self.stages)):
-                self.landing_given_up += 1
+        yield from self.land("full", self.stages, issued)
 
     def load(self):
         ok, issued = not self.failed, 0
@@ -70,7 +46,7 @@ class Cta:
             if u and not (yield from self.wait(f"empty{s}", u - 1)):
                 ok = False
                 break
-            (self.held if c in self.late else self.copies).append(f"full{s}")
+            self.copy(c, f"full{s}")
             issued = c + 1
             yield "step"
         if not ok:
@@ -117,39 +93,8 @@ class Cta:
     def run(self):
         roles = {"load": self.load(), "mma": self.mma()}
         roles.update({f"epi{w}": self.epilogue(w) for w in range(EPI)})
-        idle = 0
-        while roles:
-            if self.limits >= self.after and self.held:
-                self.copies, self.held = self.copies + self.held, []
-            names = list(roles) + (["copy"] if self.copies else []) + (["commit"] if self.commits else [])
-            n = self.rnd.choice(names)
-            if n == "copy":
-                self.arrive(self.copies.pop(self.rnd.randrange(len(self.copies))))
-                idle = 0
-                continue
-            if n == "commit":
-                self.arrive(self.commits.pop(0))
-                idle = 0
-                continue
-            try:
-                r = next(roles[n])
-            except StopIteration:
-                del roles[n]
-                idle = 0
-                continue
-            if r == "step":
-                idle = 0
-                continue
-            idle += 1
-            if idle > 40 * (2 + EPI) and not self.copies and not self.commits:
-                self.limits += 1  # nothing moves: the waits open now run out
-                self.gen += 1
-                idle = 0
-                assert self.limits < 50, "a wait without a bound"
+        self.play(roles)
         return all(self.good.values())
-
-    def in_flight(self):
-        return len(self.copies) + len(self.held)
 
 
 SHAPES = [(c, s) for s in (2, 3) for c in (1, 2, 3, 4, 5, 8)]
@@ -158,7 +103,7 @@ SHAPES = [(c, s) for s in (2, 3) for c in (1, 2, 3, 4, 5, 8)]
 @pytest.mark.parametrize("chunks, stages", SHAPES)
 def test_every_role_ends_on_a_phase_boundary(chunks, stages):
     for seed in range(20):
-        c = Cta(chunks, stages, seed)
+        c = Pipeline(chunks, stages, seed)
         assert c.run() and c.limits == 0
         assert not c.aliased and not any(c.pending.values()) and not c.in_flight() and not c.commits
 
@@ -169,9 +114,9 @@ def test_no_copy_in_flight_at_exit(chunks, stages):
     for late in range(chunks):
         for after in (1, 2):
             for seed in range(5):
-                c = Cta(chunks, stages, seed, {late}, after)
+                c = Pipeline(chunks, stages, seed, {late}, after)
                 assert not c.run()
-                assert not c.commits and c.in_flight() <= c.landing_given_up
+                assert not c.commits and c.in_flight() <= c.given_up_landing
                 if after == 1:
                     assert c.in_flight() == 0, (late, seed)
 
@@ -183,10 +128,10 @@ def test_a_failed_run_ends_promptly(chunks, stages):
     def run(reads):
         limits, failed = 0, False
         for k in range(40):
-            c = Cta(chunks, stages, k, range(chunks), 1 << 30, failed=failed and reads)
+            c = Pipeline(chunks, stages, k, range(chunks), 1 << 30, failed=failed and reads)
             failed = not c.run() or failed
             limits += c.limits
-            assert not c.commits and c.in_flight() <= c.landing_given_up
+            assert not c.commits and c.in_flight() <= c.given_up_landing
         return limits
     assert run(True) <= 1 + stages
     assert run(False) >= 40
@@ -197,7 +142,7 @@ def test_a_drain_by_the_load_lane_alone_is_caught():
     ones outlives the CTA, and the model finds it."""
     found = []
     for chunks, stages in SHAPES:
-        c = Cta(chunks, stages, 1, {chunks - 1}, 2, drain_all=False)
+        c = Pipeline(chunks, stages, 1, {chunks - 1}, 2, drain_all=False)
         assert not c.run()
-        found.append(c.in_flight() > c.landing_given_up)
+        found.append(c.in_flight() > c.given_up_landing)
     assert all(found), found
