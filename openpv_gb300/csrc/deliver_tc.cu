@@ -77,11 +77,6 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
    return reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
 }
 
-// The last of `sent` copies through a ring of `slots` barriers land (out of line: only a failing run calls it).
-__device__ __noinline__ void land(uint64_t *full, int slots, uint32_t sent) {
-   for (uint32_t c = sent > (uint32_t)slots ? sent - slots : 0; c < sent; c++) mbar_wait(&full[c % slots], (c / slots) & 1);
-}
-
 // R = target rows per unit (g.R); NCH = R * NT / 32: 32-column chunks of the result, summed in
 // registers by the epilogue (a chain buffer holds 2 * NCH chunks: hi-weight and lo-weight
 // columns).  R is a template parameter so that the 8R MMAs of one weight tile issue as one
@@ -411,8 +406,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
       atomicExch(err, 1);
       // copies still in flight must land before the CTA may exit, whichever role gave up: the producer may have
       // issued all of its own by then
-      land(rawFull, g.NR, sentA);
-      land(bFull, g.NB, sentB);
+      mbar_land(rawFull, g.NR, (int)sentA);
+      mbar_land(bFull, g.NB, (int)sentB);
    }
    tc_fence_before();
    __syncthreads();

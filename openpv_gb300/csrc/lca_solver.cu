@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(320, 1)
          xEmpty[2];
    __shared__ uint32_t tmemBase;
    __shared__ volatile int abortFlag;
+   __shared__ int allSent;  // the load lane has issued every copy
 
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    const int G = gridDim.x;
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(320, 1)
          mbar_init(&xFull[i], 1);
          mbar_init(&xEmpty[i], 1);
       }
-      abortFlag = 0;
+      abortFlag = allSent = 0;
       fence_mbar_init();
    }
    if (warp == 0) tmem_alloc(&tmemBase, 512);
@@ -177,7 +178,6 @@ __global__ void __launch_bounds__(320, 1)
       abortFlag = 1;
       return false;
    };
-   auto last_use = [](int n, int sl, int slots) { return sl < n ? n - 1 - ((n - 1 - sl) % slots) : -1; };
 
    if (warp == 8) {
       // ============================== loads ==============================
@@ -221,15 +221,9 @@ __global__ void __launch_bounds__(320, 1)
             }
          }
          if (!ok) {
-            for (int sl = 0; sl < nStage; sl++) {
-               const int u = last_use(issued, sl, nStage);
-               if (u >= 0) mbar_wait(&full[sl], (uint32_t)((u / nStage) & 1));
-            }
-            for (int sl = 0; sl < 2; sl++) {
-               const int u = last_use(xIssued, sl, 2);
-               if (u >= 0) mbar_wait(&xFull[sl], (uint32_t)((u / 2) & 1));
-            }
-         }
+            mbar_land(full, nStage, issued);
+            mbar_land(xFull, 2, xIssued);
+         } else allSent = 1;
       }
    } else if (warp == 9) {
       // ============================== MMA ==============================
@@ -362,7 +356,14 @@ __global__ void __launch_bounds__(320, 1)
       }
    }
    __syncthreads();
-   if (tid == 0 && abortFlag) atomicExch(err, 1);
+   if (tid == 0 && abortFlag) {
+      atomicExch(err, 1);
+      // another role gave up: the last copies may be what was waited for
+      if (allSent) {
+         mbar_land(full, nStage, myUnits * g.MB * nkc);
+         mbar_land(xFull, 2, myUnits);
+      }
+   }
    tc_fence_before();
    __syncthreads();
    if (warp == 0) tmem_dealloc(tmem, 512);
@@ -442,6 +443,7 @@ __global__ void __launch_bounds__(320, 1) post_tc_kernel(const __grid_constant__
          vFull[kMaxVSlots], vEmpty[kMaxVSlots], accFull[kAcc], accEmpty[kAcc];
    __shared__ uint32_t tmemBase;
    __shared__ volatile int abortFlag;
+   __shared__ int allSent;  // the load lane has issued every copy
 
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    const int nFH = g.F / pl.FT, nBlk = pl.FT / kPostNT;
@@ -470,7 +472,7 @@ __global__ void __launch_bounds__(320, 1) post_tc_kernel(const __grid_constant__
          mbar_init(&accFull[i], 1);
          mbar_init(&accEmpty[i], 8);
       }
-      abortFlag = 0;
+      abortFlag = allSent = 0;
       fence_mbar_init();
    }
    if (warp == 0) tmem_alloc(&tmemBase, kAcc * kPostNT);
@@ -496,8 +498,6 @@ __global__ void __launch_bounds__(320, 1) post_tc_kernel(const __grid_constant__
       abortFlag = 1;
       return false;
    };
-   // last block (< n issued) that used ring slot sl of a ring of `slots`, or -1
-   auto last_use = [](int n, int sl, int slots) { return sl < n ? n - 1 - ((n - 1 - sl) % slots) : -1; };
 
    if (warp == 8) {
       // ============================== loads ==============================
@@ -563,16 +563,10 @@ __global__ void __launch_bounds__(320, 1) post_tc_kernel(const __grid_constant__
          }
          if (!ok) {
             // the copies still in flight land before shared memory goes away
-            mbar_wait(&stFull, (uint32_t)((rowsIssued - 1) & 1));
-            for (int sl = 0; sl < nW; sl++) {
-               const int u = last_use(wIssued, sl, nW);
-               if (u >= 0) mbar_wait(&wFull[sl], (uint32_t)((u / nW) & 1));
-            }
-            for (int sl = 0; sl < nV; sl++) {
-               const int u = last_use(vIssued, sl, nV);
-               if (u >= 0) mbar_wait(&vFull[sl], (uint32_t)((u / nV) & 1));
-            }
-         }
+            mbar_land(&stFull, 1, rowsIssued);
+            mbar_land(wFull, nW, wIssued);
+            mbar_land(vFull, nV, vIssued);
+         } else allSent = 1;
       }
    } else if (warp == 9) {
       // ============================== MMA ==============================
@@ -801,7 +795,15 @@ __global__ void __launch_bounds__(320, 1) post_tc_kernel(const __grid_constant__
       if (lane == 0) bulk_wait_all();
    }
    __syncthreads();
-   if (tid == 0 && abortFlag) atomicExch(err, 1);
+   if (tid == 0 && abortFlag) {
+      atomicExch(err, 1);
+      // another role gave up: the last copies may be what was waited for
+      if (allSent) {
+         mbar_land(&stFull, 1, myTiles);
+         mbar_land(wFull, nW, Q);
+         mbar_land(vFull, nV, Q);
+      }
+   }
    tc_fence_before();
    __syncthreads();
    if (warp == 0) tmem_dealloc(tmem, kAcc * kPostNT);
@@ -903,6 +905,7 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
          drain;
    __shared__ uint32_t tmemBase;
    __shared__ volatile int abortFlag;
+   __shared__ int weightsSent, rowsSent;  // the load lanes have issued every weight tile, every stage and V chunk
 
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    const int nFH = g.F / fp.FT, nBlk = fp.FT / kPostNT;
@@ -941,7 +944,7 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
       mbar_init(&foldFree, 1);
       mbar_init(&xFull, 1);
       mbar_init(&drain, 1);
-      abortFlag = 0;
+      abortFlag = weightsSent = rowsSent = 0;
       fence_mbar_init();
    }
    if (warp == 0) tmem_alloc(&tmemBase, 512);
@@ -979,7 +982,6 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
       if (idle > 16) __nanosleep(32);  // leave the issue slots to the epilogue warps on this sub-partition
       return true;
    };
-   auto last_use = [](int n, int sl, int slots) { return sl < n ? n - 1 - ((n - 1 - sl) % slots) : -1; };
    auto band_in = [&](int b, int mb, int fh) {
       return rin + (((size_t)b * g.MB + mb) * nFH + fh) * fp.bandFloats;
    };
@@ -1009,11 +1011,8 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
             }
          }
          if (!ok) {  // the copies still in flight land before shared memory goes away
-            for (int sl = 0; sl < nW; sl++) {
-               const int u = last_use(wIssued, sl, nW);
-               if (u >= 0) mbar_wait(&wFull[sl], (uint32_t)((u / nW) & 1));
-            }
-         }
+            mbar_land(wFull, nW, wIssued);
+         } else weightsSent = 1;
       }
    } else if (warp == LW) {
       // ============================== V and stage loads ==============================
@@ -1080,12 +1079,9 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
          if (!ok) {
             // the copies still in flight land before shared memory goes away (a stage is issued
             // only after the one before it has landed and been read)
-            if (stNext > 0) mbar_wait(&stFull, (uint32_t)((stNext - 1) & 1));
-            for (int sl = 0; sl < nV; sl++) {
-               const int u = last_use(vq, sl, nV);
-               if (u >= 0) mbar_wait(&vFull[sl], (uint32_t)((u / nV) & 1));
-            }
-         }
+            mbar_land(&stFull, 1, stNext);
+            mbar_land(vFull, nV, vq);
+         } else rowsSent = 1;
       }
    } else if (warp == MW) {
       // ============================== MMA ==============================
@@ -1521,7 +1517,15 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
       if (lane == 0) bulk_wait_all();
    }
    __syncthreads();
-   if (tid == 0 && abortFlag) atomicExch(err, 1);
+   if (tid == 0 && abortFlag) {
+      atomicExch(err, 1);
+      // another role gave up: the last copies may be what was waited for
+      if (weightsSent) mbar_land(wFull, nW, Q);
+      if (rowsSent) {
+         mbar_land(&stFull, 1, myTiles);
+         mbar_land(vFull, nV, Q);
+      }
+   }
    tc_fence_before();
    __syncthreads();
    if (warp == 0) tmem_dealloc(tmem, 512);

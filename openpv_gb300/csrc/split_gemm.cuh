@@ -90,13 +90,6 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p) {
    return p + ((1024u - (a & 1023u)) & 1023u);
 }
 
-// The last copies of `chunks` stages land.  Out of line: a healthy run never calls it, and inlined it costs the
-// gradient 4 % through what the compiler then makes of the rest (32 x 64x64x1 -> 16x16x256, 100 steps: 11.23 ms, now
-// 10.81).
-static __device__ __noinline__ void land(uint64_t *full, int stages, int chunks) {
-   for (int c = chunks > stages ? chunks - stages : 0; c < chunks; c++) mbar_wait(&full[c % stages], (uint32_t)((c / stages) & 1));
-}
-
 // A wait of a kernel of a run: at most kWaitNs, and no longer than a look at the run's error word where it is set,
 // so that a run whose first wait gave up ends at once and not after a limit for each of its kernels.
 __device__ __forceinline__ bool run_wait(uint64_t *bar, uint32_t parity, const int *err) {
@@ -162,7 +155,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
             load(c, smem + s * stageBytes, &full[s]);
             issued = c + 1;
          }
-         if (!ok) land(full, kStages, issued);  // copies in flight land before the CTA may exit
+         if (!ok) mbar_land(full, kStages, issued);  // copies in flight land before the CTA may exit
       }
    } else if (warp == kEpiWarps + 1) {
       if (lane == 0) {
@@ -217,7 +210,7 @@ __device__ __forceinline__ void pipeline(uint8_t *smem, uint32_t stageBytes, int
    float *z = reinterpret_cast<float *>(smem);  // the stages are free: every MMA is done
    if (!good) {
       if (threadIdx.x == 0) atomicExch(err, 1);
-      if (warp == kEpiWarps && lane == 0 && ok) land(full, kStages, chunks);
+      if (warp == kEpiWarps && lane == 0 && ok) mbar_land(full, kStages, chunks);
    } else if (warp < kEpiWarps) {
       const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * BN + (warp >> 2) * HALF;
       float *zr = z + (size_t)((warp & 3) * 32 + lane) * LZ + (warp >> 2) * HALF;

@@ -78,6 +78,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
    }
 }
 
+// The last of `sent` copies through a ring of `slots` barriers land, each waited for as long as any wait: a CTA must
+// not exit with a copy in flight, whichever role gave up.  Out of line: only a failing run calls it, and inlined into
+// the split-plane GEMMs it cost the gradient 4 % through what the compiler then made of the rest (32 x 64x64x1 ->
+// 16x16x256, 100 steps: 11.23 ms, now 10.81).
+__device__ __noinline__ inline void mbar_land(uint64_t *full, int slots, int sent) {
+   for (int c = sent > slots ? sent - slots : 0; c < sent; c++) mbar_wait(&full[c % slots], (uint32_t)((c / slots) & 1));
+}
+
 // ---- TMA -------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1) {
    asm volatile(
