@@ -128,7 +128,7 @@ __device__ __forceinline__ void search_keys(const pvgpu_entry *e, int n, int key
 // Each entry is read and decoded once per warp and feeds nyp x FPL multiply-adds per lane.
 //
 // What bounds it: the weight stream.  Every (entry, weight) product is distinct, so each FMA takes
-// its own 4 bytes from L2: 8.8 GB at 17 TB/s, 71 % of L2's rate, on the delivery microbenchmark at
+// its own 4 bytes from L2: 8.2 GB at 17.4 TB/s, 71 % of L2's rate, on the delivery microbenchmark at
 // 1 % activity (0.469 ms; 0.522 ms with a test per patch row, which ran 2.7 times the instructions
 // and left the issue slots the limit).  A patch is therefore
 // added whole, also where some of its rows lie outside [P0, P1) (they are dropped when the window

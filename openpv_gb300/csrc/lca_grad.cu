@@ -14,8 +14,8 @@
 // and their adjoints (the transpose delivery and the pre (x) post-error correlation):
 //   gR = (1 - e) g . W,  gr = fold(gR),  gD = -im2col(gr),  gA = gD . W^T,
 //   g <- e g + [V >= VThresh] ((1 - e) g + gA),   dW += (1 - e) g^T R + A^T gD
-// where g = dL/dV of the later step; the correlations of a whole segment run as two GEMMs over all
-// its steps' positions (K = steps x positions).  The final loss seeds g_T = [V_T >= VThresh](-Z_T + lambda [a_T > 0])
+// where g = dL/dV of the later step; on the library path below the correlations of a whole segment run as two
+// GEMMs over all its steps' positions (K = steps x positions).  The final loss seeds g_T = [V_T >= VThresh](-Z_T + lambda [a_T > 0])
 // and dW = -A_T^T R_T.
 //
 // Where v1Nf and KP are multiples of 8 the GEMMs are the split-plane ones of split_gemm.cuh (tcgen05, six
@@ -24,12 +24,12 @@
 //   fold_im2col (residual windows gathered from D, their im2col written as planes),
 //   drive GEMM, whose epilogue updates V and writes the planes of the new activity,
 // and an adjoint step the same three plus the correlations of that step's positions, added into one
-// partial dW per range of positions.  Measured for 32 x 64x64x1 -> 16x16x256, 100 steps: 11.2 ms against
+// partial dW per range of positions.  Measured for 32 x 64x64x1 -> 16x16x256, 100 steps: 10.7 ms against
 // 16.8 ms with library GEMMs (14.4 us each, nine plane products) and separate fold, im2col and update
-// passes (31 us a step); dW's median error against FP64 over 40 inputs 1.7e-7 against 7e-7.  The last
+// passes (31 us a step); dW's median error against FP64 over 40 inputs 2.1e-7 against 6.0e-7.  The last
 // segment's states are kept from the forward pass.
 //
-// Other sizes run on cuBLAS in FP32 emulated on the BF16 tensor cores
+// Other sizes, and runs whose buffers fit in no other way, go through cuBLAS in FP32 emulated on the BF16 tensor cores
 // (CUBLAS_COMPUTE_32F_EMULATED_16BFX9: each operand split in three BF16 parts, FP32 accuracy), or
 // in plain FP32 where that mode is refused.  cuBLAS is loaded at the first create that needs it.
 // Everything else -- fold, im2col, the update and its adjoint,
@@ -340,7 +340,7 @@ __global__ void split_activity_kernel(int64_t n8, float vt, const float *__restr
 // signImg * fold(D), each pixel gathered from the positions that cover it in ascending (y, x) order (as
 // fold_kernel), staged in shared memory, then every position's patch written as planes times signOut.
 // Neighbouring bands gather the P - S rows they share twice, from L2; in exchange the image and the
-// FP32 im2col never go to memory and the pass is one launch (23 us for the two before, 9 now).
+// FP32 im2col never go to memory and the pass is one launch (23 us for the two before, 11 now).
 // SS, PP, CC: the geometry as constants, or 0.  Any other geometry takes xPer positions of a row at a time: its
 // gather is a chain of loads per pixel, so where bands are few and patches large a row is divided (3 x 56x76x3 ->
 // 14x19x8, 16x16 patches, 16 steps: 2.49 ms with whole rows, now 1.65; the library path 1.25).

@@ -73,9 +73,9 @@ struct HGeom {
 // feature's list with its lanes on 32 * EPT weights of the patch.  Zeros cost a lane's share of a load
 // instead of a step of every chain.  The next segment's loads are issued before the lists are walked.
 //
-// 32 images of 16x16x512 at 5 % against 32x32x3 errors, 8x8 patches: 92 us (46 M instructions, a
-// third of them the scan; the rest the walk, whose patches mostly hang over the image's edge and are
-// tested weight by weight); one thread per weight walking every position itself took 4.3 ms.
+// 32 images of 16x16x512 at 5 % against 32x32x3 errors, 8x8 patches: 92 us (57 M instructions, issue slots
+// 62 % busy: the scan, and the walk, where nearly every group of entries has a patch that hangs over the
+// image's edge and is tested weight by weight); one thread per weight walking every position itself took 4.3 ms.
 // W = the most warps a CTA has.  Patches whose weights take more than 16 warps at one weight a lane get up
 // to 32 warps of one or two weights a lane, with half the loads per warp and segment (the lists of a
 // segment stay at 128 KB): twice the chains in flight.  The call above: 118 us with 16 warps of two
