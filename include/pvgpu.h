@@ -423,8 +423,8 @@ pvgpu_status pvgpu_lca_grad_create(const pvgpu_lca_grad_desc *desc, pvgpu_lca_gr
 pvgpu_status pvgpu_lca_grad_destroy(pvgpu_lca_grad *g);
 pvgpu_status pvgpu_lca_grad_run(pvgpu_lca_grad *g, const float *w, const float *x, float *dW, double *loss,
                                 void *stream);
-/* Reads (synchronously) the error word of the last run: nonzero if a bounded device wait gave up, in which case
- * dW and *loss are NaN. */
+/* Reads (synchronously; after the run's stream has been synchronised) the error word of the last run: nonzero if a
+ * bounded device wait gave up, in which case dW and *loss are NaN. */
 pvgpu_status pvgpu_lca_grad_error_flag(const pvgpu_lca_grad *g, int *hostFlag);
 /* *emulatedFp32 = 1 when the GEMMs run as FP32 emulated on the BF16 tensor cores, 0 for plain FP32. */
 pvgpu_status pvgpu_lca_grad_info(const pvgpu_lca_grad *g, int *emulatedFp32);

@@ -2057,11 +2057,12 @@ struct Launcher {
                                          a.Alo, a.err);
       return e == cudaSuccess ? PVGPU_OK : pvgpu::record_cuda_error(e, "lca fused step");
    }
-   // recon CTAs that can be resident at once (one CTA per SM)
+   // recon CTAs that can be resident at once (one CTA per SM).  The shared-memory limit belongs to the kernel, which
+   // other solvers run: it is set to the budget, as in set_attrs, not to this plan's size.
    static int max_recon_ctas(const ReconPlan &rp, bool x3) {
       const void *fn = x3 ? reinterpret_cast<const void *>(recon_tc_kernel<S, P, C, true>)
                           : reinterpret_cast<const void *>(recon_tc_kernel<S, P, C, false>);
-      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rp.total) != cudaSuccess) {
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget) != cudaSuccess) {
          cudaGetLastError();
          return 0;
       }

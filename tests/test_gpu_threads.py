@@ -89,3 +89,43 @@ def test_same_kernel_from_several_threads(torch, kernel):
         t.join()
     torch.cuda.synchronize()
     assert not errors and not wrong, (errors, wrong)
+
+
+def test_solvers_made_while_another_runs(torch):
+    """One thread makes solvers of small images while another captures and runs one of large images, which takes
+    more shared memory in the same kernels."""
+    from openpv_gb300 import capi
+    w = torch.randn((64, 8, 8, 1), device="cuda")
+    w /= w.square().sum(dim=(1, 2, 3), keepdim=True).sqrt()
+    xs = [torch.randn((2, 64, 64, 1), device="cuda") for _ in range(2)]
+    big = capi.LcaSolver(2, (64, 64, 1), (32, 32, 64), 8, 0.1)
+    big.set_weights(w)
+    torch.cuda.synchronize()
+    errors, stop = [], time.monotonic() + 3.0
+
+    def run():
+        s = torch.cuda.Stream()
+        try:
+            k = 0
+            while time.monotonic() < stop and not errors:
+                big.reset(stream=s)
+                big.run(xs[k & 1], 6, 2, precision=capi.LCA_BF16, stream=s)  # another input: captured again
+                k += 1
+                s.synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(f"run: {e}")
+
+    def make():
+        try:
+            while time.monotonic() < stop and not errors:
+                capi.LcaSolver(1, (32, 32, 1), (16, 16, 64), 8, 0.1).close()
+        except Exception as e:  # noqa: BLE001
+            errors.append(f"make: {e}")
+
+    threads = [threading.Thread(target=run), threading.Thread(target=make)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors and big.error_flag() == 0, errors
