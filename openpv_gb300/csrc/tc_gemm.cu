@@ -127,9 +127,11 @@ pvgpu_status tc_gemm(const void *A, const void *B, float *C, int M, int N, int K
    if (!pvgpu::make_tmap_bf16_sw128(&tmA, A, M, K, K, kBM) ||
        !(bmn ? pvgpu::make_tmap_bf16_sw128(&tmB, B, K, N, N, kBK) : pvgpu::make_tmap_bf16_sw128(&tmB, B, N, K, K, N)))
       return PVGPU_ERR_BAD_ARG;
-   size_t smem = 2 * (size_t)(kBM * kBK * 2 + N * kBK * 2) + 1024;
+   // the limit belongs to the kernel, which other threads may be launching: always that of N = 256
+   auto bytes = [](int n) { return 2 * (size_t)(kBM * kBK * 2 + n * kBK * 2) + 1024; };
+   const size_t smem = bytes(N);
    auto fn = bmn ? tc_gemm_kernel<true> : tc_gemm_kernel<false>;
-   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(256));
    if (e != cudaSuccess) return pvgpu::record_cuda_error(e, "tc_gemm attr");
    fn<<<M / kBM, 128, smem, pvgpu::as_stream(stream)>>>(tmA, tmB, C, M, N, K, errFlag);
    PVGPU_CHECK_LAUNCH("tc_gemm");
@@ -221,8 +223,9 @@ extern "C" pvgpu_status pvgpu_tc_gemm_bf16_atmem(const void *A, const void *B, f
       return PVGPU_ERR_BAD_ARG;
    CUtensorMap tmB;
    if (!pvgpu::make_tmap_bf16_sw128(&tmB, B, N, K, K, N)) return PVGPU_ERR_BAD_ARG;
-   const size_t smem = (size_t)(K / kBK) * N * kBK * 2 + 1024;
-   cudaError_t e = cudaFuncSetAttribute(tc_gemm_atmem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   auto bytes = [](int k, int n) { return (size_t)(k / kBK) * n * kBK * 2 + 1024; };
+   const size_t smem = bytes(K, N);
+   cudaError_t e = cudaFuncSetAttribute(tc_gemm_atmem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(256, 256));
    if (e != cudaSuccess) return pvgpu::record_cuda_error(e, "tc_gemm attr");
    tc_gemm_atmem_kernel<<<M / kBM, 128, smem, pvgpu::as_stream(stream)>>>(tmB, static_cast<const uint16_t *>(A), C, M,
                                                                           N, K, errFlag);

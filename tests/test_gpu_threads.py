@@ -56,11 +56,26 @@ def scatter(torch, capi, seed, nb, n, nf):
     return make
 
 
-@pytest.mark.parametrize("kernel", ["hebbian", "scatter"])
+def gemm(torch, capi, seed, entry, n):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    a = torch.randn((128, 256), device="cuda", generator=g).bfloat16()
+    b = torch.randn((256, n) if entry == "tc_gemm_bf16_kn" else (n, 256), device="cuda", generator=g).bfloat16()
+
+    def make():
+        c, err = torch.empty((128, n), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        return lambda stream: getattr(capi, entry)(a, b, c, 128, n, 256, err, stream=stream), c
+    return make
+
+
+GEMMS = ["tc_gemm_bf16", "tc_gemm_bf16_kn", "tc_gemm_bf16_atmem"]
+
+
+@pytest.mark.parametrize("kernel", ["hebbian", "scatter"] + GEMMS)
 def test_same_kernel_from_several_threads(torch, kernel):
     from openpv_gb300 import capi
     calls = {"hebbian": lambda: [hebbian(torch, capi, 1, 56), hebbian(torch, capi, 2, 2)],
-             "scatter": lambda: [scatter(torch, capi, 1, 4, 64, 64), scatter(torch, capi, 2, 2, 32, 16)]}[kernel]()
+             "scatter": lambda: [scatter(torch, capi, 1, 4, 64, 64), scatter(torch, capi, 2, 2, 32, 16)],
+             **{e: lambda e=e: [gemm(torch, capi, 1, e, 256), gemm(torch, capi, 2, e, 128)] for e in GEMMS}}[kernel]()
     alone = []
     for c in calls:
         call, out = c()
