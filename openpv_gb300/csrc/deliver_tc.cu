@@ -208,11 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tf32x3_kernel(const __grid_c
       // uniform registers: 28 -> 21), the next tile's barrier is probed in the middle of a tile's
       // MMAs, positions advance by additions, and the abort flag is read only where a wait does not
       // find its phase.  The 128x128x256 -> 64 delivery with 7x7 patches, batch 16: 2.09 -> 1.72 ms
-      // (0.62 -> 0.75 of the pairs' rate).  Tried: core matrices of every 16th position, so that a
-      // shift moves by whole 128-byte lines (the MMA rate does not depend on it; four weight tiles
-      // instead of six: 2.27); one barrier for two or three weight tiles (1.81); the probe after the
-      // first or the last MMAs (1.72); no copies of weights at all (2.07 before, 1.77 with lane 0
-      // issuing: the copies are not what the MMAs wait for).
+      // (0.62 -> 0.75 of the pairs' rate).
       const uint64_t stepB = (2 * bBytes) >> 4;
       uint32_t cc = 0;      // chains so far
       int slotA = 0;        // slot and phase of split row ky (the next one to lose its last use)

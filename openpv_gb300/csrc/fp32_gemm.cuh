@@ -25,11 +25,9 @@ namespace cg = cooperative_groups;
 // memory in rank order.
 //
 // What bounds it: shared-memory and FMA cycles about equally for large layers, 44 TFLOP/s of the
-// 66 that a register-only loop of the same FMAs reaches (M = 32,768, N = 64, K = 12,544); for one
-// image the length of the K loop, which the division over a cluster cuts.  8 x 8 per thread gained
-// 8 % at K = 12,544 and lost 18 % at K = 192 (too few warps); operands laid out [k][row] with
-// unpacked FMAs reached 0.8 of this.  Before: 64 x 64 tiles, 4 x 4 per thread, one register-staged
-// buffer, 13 to 19 TFLOP/s.
+// 66 that a register-only loop of the same FMAs reaches (M = 32,768, N = 64, K = 12,544; 13 to 19 with 64 x 64
+// tiles of 4 x 4 per thread and one register-staged buffer); for one image the length of the K loop, which the
+// division over a cluster cuts.
 constexpr int BK = 16, LDK = BK + 4, kStages = 4;
 
 template <int VW>
